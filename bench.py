@@ -363,7 +363,14 @@ def roofline_of(tm, a, fp64_rate, fp32_rates, split):
                   "per object: 8 B key read, 32 B FP32 record gathered, 32 B record + 4 B index written"),
         "pairs": (32.0 * n_obj, phases["pairs_ms"], "per object: its 32 B FP32 record read once"),
     }
-    if tm.get("sort_cells_fused"):
+    if tm.get("sort_cells_fused") == 2:
+        hbm_phases = {
+            "cells": (92.0 * n_obj, phases["sort_ms"] + phases["cells_ms"],
+                      "per object: 8 B key read, 8 B place written and read, 32 B FP32 record read and written, "
+                      "4 B index written"),
+            "pairs": hbm_phases["pairs"],
+        }
+    elif tm.get("sort_cells_fused"):
         # One launch sorts and builds the cells: its time is the sort phase's.
         hbm_phases = {
             "sort_cells": ((16.0 * passes + 76.0) * n_obj, phases["sort_ms"] + phases["cells_ms"],
@@ -430,10 +437,13 @@ def traffic_of(kernel, split):
 
 
 def launches_per_step(sort_passes, fused=False):
+    # Counted cells (2): propagate, place, number, scatter, cells, pairs, refine.
     # Fused: propagate, fix_keys, sort + cells (one cooperative launch), pairs,
     # refine. Otherwise: propagate, fix_keys, sort (one kernel per pass; the
     # propagation and, if it rebuilds keys, k_fix_keys count the digits), cells
     # (count, scan, write, neighbours, item count, scan, item write), pairs, refine.
+    if fused == 2:
+        return 1 + 4 + 1 + 1
     if fused:
         return 1 + 1 + 1 + 1 + 1
     return 1 + 1 + sort_passes + 7 + 1 + 1
@@ -557,7 +567,7 @@ def main():
                 "exact_filter_pairs_per_step": tm["exact_filter_pairs"] / steps,
                 "roofline": roofline_of(tm, a, fp64_rate, fp32_rate, prec == ks.PRECISION_SPLIT),
                 "wall_s_timed_region": wall, "sort_passes": tm["sort_passes"],
-                "sort_cells_fused": bool(tm.get("sort_cells_fused", 0))}
+                "sort_cells_fused": int(tm.get("sort_cells_fused", 0))}
 
     main_s, other_s = summary(head), summary(other)
     c_head, c_other = runs[head][1], runs[other][1]

@@ -123,7 +123,10 @@ int ks_set_l2_flush(ks_ctx* ctx, int64_t bytes);
  * FP64 propagation kernel is compiled for; more blocks, fewer registers each),
  * "sort_rank_ballot" (radix-sort ranking within a warp: 0, the default, by
  * the hardware match instruction; 1 by eight ballots, one per digit bit),
- * "sort_fused" (1, the default: the object sort and the cell build run as one
+ * "sort_fused" (2, the default: cells built by counting - every object finds or
+ * opens its cell in a hash and takes its place in the cell by its order of
+ * arrival, nothing is sorted - wherever the keys carry the object index and the
+ * pair kernel gates in FP32; 1: the object sort and the cell build run as one
  * cooperative launch of one 1024-thread block per SM, grid barriers between
  * their phases, wherever the keys fit its registers (up to 12 288 per SM) and
  * the keys carry the object index; 0: the separate radix passes and cell
@@ -314,8 +317,9 @@ typedef struct ks_timing {
     int64_t refined_pairs;       /* pairs refined (Hermite TCA) */
     double chunk_ms;       /* device work of the chunks outside their steps: set-up, checkpoint,
                               ordering of the chunk's conjunction records, replays (L2 flushes excluded) */
-    int64_t sort_cells_fused;  /* 1: the last steps sorted and built the cells in one cooperative launch
-                                  (sort_ms then holds both, cells_ms is 0); 0: separate kernels */
+    int64_t sort_cells_fused;  /* the last steps' cell build ("sort_fused"): 2 by counting (cells_ms; sort_ms is 0),
+                                  1 sort and build in one cooperative launch (sort_ms holds both, cells_ms is
+                                  0), 0 separate kernels */
     /* Host wall time of the run's chunks (fragmentation on the host), always
      * measured: in all, before the first launch of each chunk (parameters,
      * buffer sizing, graph capture), in the launch calls, waiting for the

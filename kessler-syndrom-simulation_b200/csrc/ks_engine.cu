@@ -149,6 +149,7 @@ void free_objects(ks_ctx* ctx) {
     dfree(b.size_m); dfree(b.real_id); dfree(b.ckpt_state); dfree(b.ckpt_alive); dfree(b.block_counts);
     dfree(b.sort_hist); dfree(b.sort_status); dfree(b.sort_ctr);
     dfree(b.cell_begin); dfree(b.cell_key); dfree(b.nbr); dfree(b.cell_len); dfree(b.col_tab); dfree(b.item_part); dfree(b.hash_keys); dfree(b.hash_vals);
+    dfree(b.place); dfree(b.span); dfree(b.cell_span); dfree(b.occ);
     dfree(b.sorted); dfree(b.sorted32); dfree(b.rec32); dfree(b.sorted_orig); dfree(b.fused);
     b.fused_grid = 0;
     dfree(b.n_live); dfree(b.mass_kg); dfree(b.a2m); dfree(b.event_of); dfree(b.coll); dfree(b.sbm_work);
@@ -199,6 +200,11 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     b.hash_cap = h;
     KS_CUDA(cudaMalloc(&b.hash_keys, sizeof(unsigned long long) * h));
     KS_CUDA(cudaMalloc(&b.hash_vals, sizeof(int) * h));
+    KS_CUDA(cudaMalloc(&b.place, sizeof(int2) * cap));
+    KS_CUDA(cudaMalloc(&b.span, sizeof(int2) * h));
+    KS_CUDA(cudaMalloc(&b.cell_span, sizeof(int2) * cap));
+    KS_CUDA(cudaMalloc(&b.occ, sizeof(unsigned long long) * (h / 4)));
+    KS_CUDA(cudaMemset(b.occ, 0, sizeof(unsigned long long) * (h / 4)));
     KS_CUDA(cudaMalloc(&b.sorted, sizeof(double) * 6 * cap));
     KS_CUDA(cudaMalloc(&b.sorted32, sizeof(float4) * 2 * cap));
     KS_CUDA(cudaMalloc(&b.rec32, sizeof(float4) * 2 * cap));
@@ -432,13 +438,15 @@ StepArgs step_args(ks_ctx* ctx, int k, int k_steps, int src) {
         a.pack_bits = ctx->pack_keys ? index_bits(ctx->b.cap) : 0;
     }
     // The fused sort counts its own digits: the propagation need not.
-    if (a.hist && ks::sort_cells_fused(ctx->b, a)) a.hist = nullptr;
+    if (a.hist && (ks::cells_counted(ctx->b, a) || ks::sort_cells_fused(ctx->b, a))) a.hist = nullptr;
     return a;
 }
 
-// Which cell build the steps take: 0 separate kernels, 1 the fused launch.
+// Which cell build the steps take: 0 separate kernels, 1 the fused launch, 2 by counting.
 int fused_form(ks_ctx* ctx) {
-    return ctx->screening && ks::sort_cells_fused(ctx->b, step_args(ctx, 0, 1, 0)) ? 1 : 0;
+    if (!ctx->screening) return 0;
+    const StepArgs a = step_args(ctx, 0, 1, 0);
+    return ks::cells_counted(ctx->b, a) ? 2 : ks::sort_cells_fused(ctx->b, a) ? 1 : 0;
 }
 
 ks::SbmArgs sbm_args(const ks_ctx* ctx) {
@@ -483,12 +491,17 @@ void enqueue_chunk(ks_ctx* ctx, int k_steps, int src0, bool capturing) {
         ks::launch_propagate(ctx->b, a, s);
         record(ctx, k, 1, capturing);
         if (ctx->screening) {
-            ks::launch_fix_keys(ctx->b, a, s);
-            if (ks::sort_cells_fused(ctx->b, a)) {
+            if (ks::cells_counted(ctx->b, a)) {
+                record(ctx, k, 2, capturing);
+                ks::launch_count_cells(ctx->b, a, false, s);  // no sort: timed as the cells
+                record(ctx, k, 3, capturing);
+            } else if (ks::sort_cells_fused(ctx->b, a)) {
+                ks::launch_fix_keys(ctx->b, a, s);
                 ks::launch_sort_cells(ctx->b, a, s);  // sort and cells in one launch: timed as the sort
                 record(ctx, k, 2, capturing);
                 record(ctx, k, 3, capturing);
             } else {
+                ks::launch_fix_keys(ctx->b, a, s);
                 ks::launch_sort(ctx->b, a, s);
                 record(ctx, k, 2, capturing);
                 ks::launch_cells(ctx->b, a, s);
@@ -1559,7 +1572,7 @@ int ks_set_tuning(ks_ctx* ctx, const char* key, int64_t value) {
         ctx->tune.sort_digit_bits = static_cast<int>(value);
         drop_graphs(ctx);
     }
-    else if (k == "sort_fused" && (value == 0 || value == 1)) {
+    else if (k == "sort_fused" && value >= 0 && value <= 2) {
         ctx->tune.sort_fused = static_cast<int>(value);
         drop_graphs(ctx);
     }

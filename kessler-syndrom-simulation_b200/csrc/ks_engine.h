@@ -90,7 +90,10 @@ struct Ctrl {
     unsigned long long exact_evals;    // candidates that needed the full filter
     int n_alive;                       // alive after the step
     int n_cells;
-    unsigned int n_items;              // pair work items
+    unsigned int n_items;              // pair work items (counted build: those at the front of the list)
+    unsigned int n_items_back;         // counted build: items at the back of the list
+    unsigned int n_tabs;               // counted build: column tables written
+    unsigned long long placed;         // counted build: objects placed << 32 | cells
     unsigned int item_ticket;          // next pair work item to hand out
     int max_cell;
     int flags;
@@ -99,7 +102,7 @@ struct Ctrl {
 };
 
 // Pair work items of a step.
-inline int64_t items_total(const Ctrl& c) { return static_cast<int64_t>(c.n_items); }
+__host__ __device__ inline int64_t items_total(const Ctrl& c) { return static_cast<int64_t>(c.n_items) + c.n_items_back; }
 
 struct ChunkCtrl {
     int halt_step;                     // device SBM: first step of the chunk left void (-1: none); later steps did nothing
@@ -139,6 +142,11 @@ struct DeviceBuffers {
     unsigned long long* hash_keys = nullptr;
     int* hash_vals = nullptr;
     int64_t hash_cap = 0;                  // power of two
+    // Counted cell build (null in the allocation-free entry point, which sorts).
+    unsigned long long* occ = nullptr;     // occupancy words, a quarter of the hash slots (all zero between steps)
+    int2* place = nullptr;                 // per object: its cell's slot, rank in it
+    int2* cell_span = nullptr;             // per cell: first sorted position and objects
+    int2* span = nullptr;                  // per slot: first sorted position and objects of its cell
     double* sorted = nullptr;              // 6 per sorted entry
     float4* sorted32 = nullptr;            // FP32 records: cell-relative position, velocity, in cell order
     float4* rec32 = nullptr;               // the same records in object order, written with the keys
@@ -191,7 +199,8 @@ struct Tuning {
     int pair_stage2 = 1;          // second FP32 stage: 0 row by row, 1 compacted when sparse, 2 always compacted
     int sort_rank_ballot = 0;     // radix ranking by eight ballots instead of the hardware match
     int prop_min_blocks = 4;      // FP64 propagation: resident 128-thread blocks per SM it is compiled for (4..6)
-    int sort_fused = 1;           // object sort and cell build in one cooperative launch (k_sort_cells) where it fits
+    int sort_fused = 2;           // cell build: 2 by counting where it fits, 1 sort and build in one cooperative launch
+                                  // (k_sort_cells) where it fits, 0 separate sort and cell kernels
     int sort_digit_bits = 8;      // fused sort: 8-bit digits; 11: 11-bit digits where they save a pass and fit
     int hash_slots_per_cell = 0;  // fused cell build: 0 packed buckets (4 slots a cell) where keys fit, else the whole
                                   // table; n: (key, cell) pairs over n slots a cell (rounded to a power of two)
@@ -311,6 +320,10 @@ int fused_grid();
 int64_t fused_scratch_words(int grid);
 bool sort_cells_fused(const DeviceBuffers& b, const StepArgs& a);
 void launch_sort_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
+// Counted cell build: whether a step takes it; its launches in place of
+// launch_fix_keys, launch_sort and launch_cells (screen: of launch_screen_keys too).
+bool cells_counted(const DeviceBuffers& b, const StepArgs& a);
+void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, cudaStream_t stream);
 void launch_pairs(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 // Orders the chunk's conjunction records by TCA into conj_sorted (records
 // whose TCAs share a 32-bit key keep their append order; the host finishes

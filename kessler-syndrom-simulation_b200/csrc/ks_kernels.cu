@@ -6,6 +6,10 @@
 //               cell key from the start-of-step position and reduces the speed and
 //               position bounds that define the next step's grid
 //   fix_keys    recomputes keys only when an object that held the top speed died
+//   cells       objects counted into cells through a hash and placed cell by
+//               cell, the cells' forward neighbours, sparse cells screened at
+//               once, work items for the others (k_place .. k_cells); or, where
+//               that does not apply or is not asked for:
 //   sort        LSD radix sort of (key, index), 8-bit digits, only over the key
 //               bits the compact key layout needs
 //   cells       cell ranges, open-addressing hash of cell keys, 13 forward
@@ -340,7 +344,8 @@ __device__ void ctrl_reset(Ctrl& c) {
     c.vmax_true = 0ull;
     c.candidates = c.co_orbiting = c.refined = c.conj = c.object_steps = c.exact_evals = 0ull;
     c.n_alive = c.n_cells = c.max_cell = c.flags = 0;
-    c.n_items = 0u;
+    c.n_items = c.n_items_back = c.n_tabs = 0u;
+    c.placed = 0ull;
     c.item_ticket = 0u;
     c.n_coll = 0u;
     c.grid = GridParams{};
@@ -734,6 +739,26 @@ __device__ __forceinline__ unsigned int block_exclusive_scan(unsigned int v, uns
     if (lane == 31) wsum[warp] = incl;
     __syncthreads();
     unsigned int off = 0, tot = 0;
+    for (int w = 0; w < kWarps; ++w) {
+        if (w < warp) off += wsum[w];
+        tot += wsum[w];
+    }
+    __syncthreads();
+    *total = tot;
+    return off + incl - v;
+}
+
+__device__ __forceinline__ unsigned long long block_exclusive_scan_u64(unsigned long long v, unsigned long long* total) {
+    __shared__ unsigned long long wsum[kWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    unsigned long long off = 0, tot = 0;
     for (int w = 0; w < kWarps; ++w) {
         if (w < warp) off += wsum[w];
         tot += wsum[w];
@@ -1895,6 +1920,32 @@ __device__ __forceinline__ void exact_rows_f32(unsigned need, float4 cp, float4 
     queue_exact<true>(still, q, fq, fcount, before, orig, nullptr, rorig, a, surv, surv_cap, pc);
 }
 
+// What the FP32 tests compare with, for the step's grid and speeds.
+struct PairGate {
+    float er, ev;        // error bounds of the FP32 records (f32_pos_err, f32_vel_err)
+    float gate, gate2;   // the exact filter's distance gate widened by er + ev dt, and its square
+    float vmin2e;        // (minimum encounter speed + ev)^2
+    float dt, cell;
+};
+
+__device__ __forceinline__ PairGate pair_gate(const StepArgs& a) {
+    const double vmax = __longlong_as_double(static_cast<long long>(a.ctrl->vmax_true));
+    const double dt3 = a.dt * a.dt * a.dt;
+    const double gate_hi = (a.threshold_km + kGravityGradient * (2.0 * vmax) * dt3 + 1e-3) * (1.0 + 1e-9);
+    const double er_d = f32_pos_err(a.ctrl->grid.cell), ev_d = f32_vel_err(vmax);
+    const double gate_e = (gate_hi + er_d + ev_d * a.dt) * (1.0 + 1e-6);
+    const double vme = sqrt(a.vmin2) + ev_d;
+    PairGate g;
+    g.er = static_cast<float>(er_d);
+    g.ev = static_cast<float>(ev_d);
+    g.gate = static_cast<float>(gate_e);
+    g.gate2 = g.gate * g.gate;
+    g.vmin2e = static_cast<float>(vme * vme * (1.0 + 1e-6));
+    g.dt = static_cast<float>(a.dt);
+    g.cell = static_cast<float>(a.ctrl->grid.cell);
+    return g;
+}
+
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kBlock, kMinBlocks) k_pairs_split(StepArgs a, const double* __restrict__ before,
                                                         const float4* __restrict__ sorted32,
@@ -1916,29 +1967,25 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_pairs_split(StepArgs a, 
     if (step_void(a.ctrl)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lanes_below = (1u << lane) - 1u;
-    const int n_items = static_cast<int>(min(static_cast<int64_t>(a.ctrl->n_items), items_cap));
-    const double vmax = __longlong_as_double(static_cast<long long>(a.ctrl->vmax_true));
-    const double dt3 = a.dt * a.dt * a.dt;
-    const double gate_hi = (a.threshold_km + kGravityGradient * (2.0 * vmax) * dt3 + 1e-3) * (1.0 + 1e-9);
-    // Error bounds of the FP32 records for this grid and these speeds.
-    const double er_d = f32_pos_err(a.ctrl->grid.cell), ev_d = f32_vel_err(vmax);
-    const float er = static_cast<float>(er_d), ev = static_cast<float>(ev_d);
-    const double gate_e = (gate_hi + er_d + ev_d * a.dt) * (1.0 + 1e-6);
-    const float gate_f = static_cast<float>(gate_e);
-    const float gate2 = gate_f * gate_f;
+    // Items of the list's front, then those of its back (counted cell build).
+    const int n_front = static_cast<int>(min(static_cast<int64_t>(a.ctrl->n_items), items_cap));
+    const int n_items = n_front + static_cast<int>(min(static_cast<int64_t>(a.ctrl->n_items_back), items_cap - n_front));
+    const int back_top = static_cast<int>(items_cap) - 1 + n_front;  // item t of the back is at back_top - t
+    // Warps beyond the number of items are not needed: they leave without a
+    // ticket (each ticket of a whole grid's first round waits on one address).
+    if (static_cast<int>(blockIdx.x * kWarps) + warp >= n_items) return;
+    const PairGate pg = pair_gate(a);
+    const float er = pg.er, ev = pg.ev, gate_f = pg.gate, gate2 = pg.gate2, dt_f = pg.dt, cell_f = pg.cell,
+                vmin2e = pg.vmin2e;
     const float2 gate2x2 = make_float2(gate2, gate2);
     const bool gate_x2 = a.tune.pair_gate_x2 != 0;
-    const float dt_f = static_cast<float>(a.dt);
-    const float cell_f = static_cast<float>(a.ctrl->grid.cell);
-    const double vme = sqrt(a.vmin2) + ev_d;
-    const float vmin2e = static_cast<float>(vme * vme * (1.0 + 1e-6));
     const int box_rows = a.tune.box_min_rows;
     const int last_record = max(0, a.ctrl->n_alive - 1);
     PairCounters pc;
     int fcount = 0;
     // Items are handed out dynamically: their costs differ by orders of magnitude.
     for (int it = next_item(a.ctrl); it < n_items; it = next_item(a.ctrl)) {
-        const int4 item = items[it];
+        const int4 item = items[it < n_front ? it : back_top - it];
         const int c = item.x, ra = item.y & 0xFFFFFF, cb0 = item.z, b0 = item.w;
         const int ncb = static_cast<int>(static_cast<unsigned int>(item.y) >> 24);
         const int r0 = 32 * ra;
@@ -2100,8 +2147,17 @@ __global__ void __launch_bounds__(kBlock) k_refine_exact(StepArgs a, const doubl
                                                          const double* __restrict__ size_m,
                                                          const int2* __restrict__ surv, int64_t surv_cap,
                                                          ks_conjunction* __restrict__ out, int64_t cap,
-                                                         ChunkCtrl* chunk) {
+                                                         ChunkCtrl* chunk, unsigned long long* __restrict__ hk,
+                                                         unsigned long long* __restrict__ occ, int64_t slots) {
     if (step_void(a.ctrl)) return;
+    // The counted build's hash and occupancy words, no longer read, left
+    // empty for the next step (slots 0: another build, which empties the hash
+    // itself).
+    for (int64_t q = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; q < slots / 2;
+         q += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        reinterpret_cast<ulonglong2*>(hk)[q] = make_ulonglong2(kEmpty, kEmpty);
+        if (q < slots / 8) reinterpret_cast<ulonglong2*>(occ)[q] = make_ulonglong2(0, 0);
+    }
     const unsigned long long ns = min(a.ctrl->refined, static_cast<unsigned long long>(surv_cap));
     const double t0 = a.sp->t0;
     const double s_hi = xsub(1.0, 1e-9);
@@ -3026,6 +3082,538 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sort_cells(StepArgs a, Fus
 }
 
 
+// ---------------------------------------------------------------------------
+// Cell build by counting (tuning "sort_fused" 2, the default; see
+// cells_counted for the rule)
+//
+// The pair kernels need the objects of a cell side by side, not the cells in
+// any order: plain launches place them without a sort.
+//   k_place    every object alive after the step finds or opens its cell's
+//              slot in the hash and takes its rank among the slot's objects
+//   k_number   one pass over the slots: room for each cell's objects (a scan
+//              and one atomic per block), and the list of the cells
+//   k_scatter  the objects' FP32 records to their places
+//   k_cells    a warp per 32 cells: their forward neighbours (occupancy words
+//              say which of the 13 to look up; the lookups are spread over
+//              the lanes); cells with few candidate pairs are screened at
+//              once, the others get their column table and work items for the
+//              tile kernel
+// A radix sort of the keys is a dozen grid barriers whatever n is, and a warp
+// per one-object cell is nearly all latency: at the catalogue's 28 340 objects
+// (26 000 cells, 49 000 candidate pairs) sort + cells + pairs took 83 + 27 us a
+// step and take 27 + 6; a batch of 64 such populations (2.13M objects, too
+// many for the cooperative sort's registers) 766 + 1400 us, now 400 + 365.
+// Every launch is bound by the latency of its few dependent L2 accesses at
+// small n and by L2 atomics and random sectors at large n (4-5% of DRAM). With
+// 1M objects in 88 000 cells both builds take about as long (110 against 130
+// us, the tile kernel 220 against 208: objects arrive in a cell in no spatial
+// order).
+// ---------------------------------------------------------------------------
+
+// Candidate pairs up to which a cell is screened by its own lanes.
+constexpr int kLightPairs = 32;
+
+struct CountArgs {
+    unsigned long long* keys;
+    unsigned long long* hk;
+    unsigned long long slots;   // hash slots in use this step, a power of two
+    int cbits;                  // low bits of an entry: the cell's objects; above them its key
+    unsigned long long* occ;    // occupancy words (all zero between steps)
+    int shift;                  // fib_slot's shift for the slots' buckets and for the occupancy words
+    int2* place;                // per object: its cell's slot (-1: dead), rank in it
+    int2* span;                 // per slot: first sorted position and objects of its cell
+    unsigned long long* cell_key;  // per cell, in no order: its key
+    int2* cell_span;            // per cell: as span
+    int* sorted_orig;
+    float4* sorted32;
+    float4* rec32;
+    int2* col_tab;
+    int4* items;
+    int64_t items_cap;
+    int per;
+};
+
+// Bucket or occupancy word of a key (Fibonacci hashing; shift is 64 less the
+// table's index bits). These kernels run a few microseconds with cold
+// instruction caches: a short instruction stream counts for more than the
+// spread of a full mixer.
+__device__ __forceinline__ unsigned long long fib_slot(unsigned long long key, int shift) {
+    return (key * 0x9E3779B97F4A7C15ull) >> shift;
+}
+
+// Occupancy words: word w of keys B = key >> 5 covers the 64 keys from
+// 32 B - 16, so that key - 1, key and key + 1 lie in one word, and each cell
+// sets its bit in two. Different B may share a word: a set bit says "look the
+// cell up", a clear one "no such cell".
+__device__ __forceinline__ void occ_set(unsigned long long* occ, int shift, unsigned long long key) {
+    const unsigned long long b = (key + 16) >> 5;
+    const unsigned bit = static_cast<unsigned>(key + 16) & 31u;
+    atomicOr(occ + fib_slot(b, shift), 1ull << bit);
+    atomicOr(occ + fib_slot(b - 1, shift), 1ull << (bit + 32));
+}
+
+// Counts one more object of the cell `key`, opening it if new: its slot and
+// the object's rank; slot -1 if the table is full (it never is: it holds more
+// slots than objects). Buckets of four slots, one 32-byte sector each, left
+// for the next bucket only when full; key and count share an entry, so that an
+// object takes one read and one atomic of one sector. The empty slot tried
+// first depends on the key: a small population's objects all arrive at once,
+// and in slot order most of them would lose the first exchange.
+__device__ __forceinline__ int2 cell_join(const CountArgs& f, unsigned long long key, bool* opened) {
+    const unsigned long long bmask = f.slots / 4 - 1, cmask = (1ull << f.cbits) - 1;
+    unsigned long long bk = fib_slot(key, f.shift);
+    const int start = static_cast<int>(fib_slot(key, f.shift - 2)) & 3;
+#pragma unroll 1
+    for (unsigned long long probe = 0; probe <= bmask;) {
+        unsigned long long s[4];
+        ld_bucket_cg(f.hk + 4 * bk, s);
+        // The slot to use is chosen before any atomic, so that the lanes of a
+        // warp, each in another bucket, take their atomics together: the
+        // cell's slot, else the first empty one.
+        unsigned free = 0, same = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (s[j] == kEmpty) free |= 1u << j;
+            else if ((s[j] >> f.cbits) == key) same |= 1u << j;
+        }
+        const bool empty = same == 0;
+        int at = -1;
+        if (same) at = __ffs(same) - 1;
+        else if (free) at = ((__ffs((free | (free << 4)) >> start) - 1) + start) & 3;
+        if (at < 0) {  // a full bucket without the key: the next one
+            bk = (bk + 1) & bmask;
+            ++probe;
+            continue;
+        }
+        unsigned long long* p = f.hk + 4 * bk + at;
+        if (empty) {
+            const unsigned long long was = atomicCAS(p, kEmpty, (key << f.cbits) | 1ull);
+            if (was == kEmpty) {
+                *opened = true;
+                return make_int2(static_cast<int>(4 * bk + at), 0);
+            }
+            if ((was >> f.cbits) != key) continue;  // taken by another cell meanwhile: look again
+        }
+        return make_int2(static_cast<int>(4 * bk + at), static_cast<int>(atomicAdd(p, 1ull) & cmask));
+    }
+    return make_int2(-1, 0);
+}
+
+// Key and FP32 record of object i made anew (out of line: the rare case must
+// not take registers from k_place's common one).
+__device__ __noinline__ unsigned long long remade_key(const GridParams& g, const double* before, int i, unsigned rid,
+                                                      float4* rec32, int* bad) {
+    double s[6];
+    ld6(before, i, s);
+    const unsigned long long key = cell_key(g, s[0], s[1], s[2], rid, bad);
+    f32_record(g, key, s[0], s[1], s[2], s[3], s[4], s[5], rec32 + 2 * static_cast<int64_t>(i));
+    return key;
+}
+
+// kScreen: one-shot screening; the keys are computed here from the given
+// states (the speculated grid is the true one), and the objects counted.
+template <bool kScreen>
+__global__ void __launch_bounds__(kBlock, kScreen ? 4 : 8) k_place(StepArgs a, CountArgs f, const double* __restrict__ before,
+                                                  const uint8_t* __restrict__ alive_after) {
+    Ctrl* ctrl = a.ctrl;
+    if (step_void(ctrl)) return;
+    const int n = live_n(a);
+    __shared__ GridParams g;
+    // When an object holding the top start speed re-entered during the step,
+    // the grid of the reference (speeds of objects alive after the step,
+    // src/core/collision.cpp:339-356) is smaller than the speculated one: the
+    // keys are made anew with it.
+    const unsigned long long vt = kScreen ? ctrl->spec_vmax : ctrl->vmax_true;
+    const bool make = kScreen || vt != ctrl->spec_vmax;
+    if (threadIdx.x == 0) {
+        if (make) {
+            make_grid(__longlong_as_double(static_cast<long long>(vt)), ctrl->bb_min, ctrl->bb_max, a.dt,
+                      a.threshold_km, a.tune.subcell_bits, a.rbits, a.tune.cell_scale, g);
+            if (blockIdx.x == 0) {
+                ctrl->grid = g;
+                if (kScreen) ctrl->vmax_true = vt;
+                check_pack_width(g, a.pack_bits, ctrl);
+            }
+        } else {
+            g.sub = ctrl->grid.sub;
+        }
+    }
+    __syncthreads();
+    const int shift = 3 * g.sub;
+    int bad = 0, alive = 0;
+    for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
+        int2 out = make_int2(-1, 0);
+        if (alive_after[i]) {
+            unsigned long long key;
+            if (make) {
+                key = remade_key(g, before, i, a.real_id ? a.real_id[i] : 0u, f.rec32, &bad);
+                ++alive;
+            } else {
+                key = f.keys[i] >> a.pack_bits;
+            }
+            key >>= shift;
+            bool opened = false;
+            out = cell_join(f, key, &opened);
+            if (opened) occ_set(f.occ, f.shift, key);
+        }
+        f.place[i] = out;
+    }
+    if (!make) return;
+    alive = warp_sum(alive);
+    bad = warp_max(bad);
+    if ((threadIdx.x & 31) == 0) {
+        if (kScreen && alive) atomicAdd(&ctrl->n_alive, alive);
+        if (bad) atomicOr(&ctrl->flags, FLAG_KEY_RANGE);
+    }
+}
+
+// Four slots (one bucket) per thread.
+__global__ void __launch_bounds__(kBlock, 6) k_number(StepArgs a, CountArgs f) {
+    Ctrl* ctrl = a.ctrl;
+    if (step_void(ctrl)) return;
+    __shared__ unsigned long long base_sh;
+    const int64_t buckets = static_cast<int64_t>(f.slots / 4);
+    const unsigned long long cmask = (1ull << f.cbits) - 1;
+    unsigned int biggest = 0;
+    for (int64_t blk = static_cast<int64_t>(blockIdx.x) * kBlock; blk < buckets; blk += static_cast<int64_t>(gridDim.x) * kBlock) {
+        const int64_t q = blk + threadIdx.x;
+        unsigned long long e[4] = {kEmpty, kEmpty, kEmpty, kEmpty};
+        if (q < buckets) ld_bucket_cg(f.hk + 4 * q, e);
+        unsigned int k[4], objects = 0, used = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            k[j] = e[j] == kEmpty ? 0u : static_cast<unsigned int>(e[j] & cmask);
+            objects += k[j];
+            used += k[j] > 0;
+        }
+        // Objects above, cells below: one scan (a block's cells and objects fit 32 bits each).
+        unsigned long long total;
+        const unsigned long long at = block_exclusive_scan_u64(
+            (static_cast<unsigned long long>(objects) << 32) | used, &total);
+        if (threadIdx.x == 0) base_sh = total ? atomicAdd(&ctrl->placed, total) : 0ull;
+        __syncthreads();
+        if (used) {
+            unsigned int b0 = static_cast<unsigned int>((base_sh + at) >> 32);
+            unsigned int ord = static_cast<unsigned int>(base_sh + at);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (k[j] == 0) continue;
+                const int2 sp = make_int2(static_cast<int>(b0), static_cast<int>(k[j]));
+                f.span[4 * q + j] = sp;
+                f.cell_key[ord] = e[j] >> f.cbits;
+                f.cell_span[ord++] = sp;
+                b0 += k[j];
+                biggest = max(biggest, k[j]);
+            }
+        }
+        __syncthreads();
+    }
+    biggest = warp_max(biggest);
+    if ((threadIdx.x & 31) == 0 && biggest > 0) atomicMax(&ctrl->max_cell, static_cast<int>(biggest));
+}
+
+__global__ void __launch_bounds__(kBlock) k_scatter(StepArgs a, CountArgs f) {
+    if (step_void(a.ctrl)) return;
+    const int n = live_n(a);
+    for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
+        const int2 pl = f.place[i];
+        if (pl.x < 0) continue;
+        const Rec32 r = ld_rec32(f.rec32 + 2 * static_cast<int64_t>(i));
+        const int p = f.span[pl.x].x + pl.y;
+        if (p < 0 || p >= n) continue;
+        f.sorted_orig[p] = i;
+        st_rec32(f.sorted32 + 2 * static_cast<int64_t>(p), r);
+    }
+}
+
+// Slot of the cell `key`, or -1.
+__device__ __forceinline__ int cell_find(const CountArgs& f, unsigned long long key) {
+    const unsigned long long bmask = f.slots / 4 - 1;
+    unsigned long long bk = fib_slot(key, f.shift);
+#pragma unroll 1
+    for (unsigned long long probe = 0; probe <= bmask; ++probe) {
+        unsigned long long s[4];
+        ld_bucket_cg(f.hk + 4 * bk, s);
+        int at = -1;
+        bool full = true;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (s[j] == kEmpty) full = false;
+            else if ((s[j] >> f.cbits) == key) at = j;
+        }
+        if (at >= 0) return static_cast<int>(4 * bk + at);
+        if (!full) return -1;
+        bk = (bk + 1) & bmask;  // a full bucket without the key: the next one
+    }
+    return -1;
+}
+
+// One pair of a light cell: the FP32 gate and second stage of k_pairs_split,
+// then the exact filter on the FP64 states.
+__device__ __forceinline__ void light_pair(const StepArgs& a, const PairGate& pg, const Rec32& col, const Rec32& row, int cp,
+                                           int rp, const double* __restrict__ before, const int* __restrict__ orig,
+                                           int2* __restrict__ surv, int64_t surv_cap, unsigned int& co,
+                                           unsigned int& full) {
+    if (!gate_open_f32(col.p, col.v, row.p, row.v, pg.gate2)) return;
+    if (certainly_reject_f32(col.p.x - row.p.x, col.p.y - row.p.y, col.p.z - row.p.z, col.v.x - row.v.x,
+                             col.v.y - row.v.y, col.v.z - row.v.z, pg.vmin2e, pg.er, pg.ev, pg.dt, pg.gate2))
+        return;
+    const int ro = orig[rp], c = orig[cp];
+    const SortedState cs = load_sorted(before, c), rs = load_sorted(before, ro);
+    ++full;
+    const int res = filter_pair_exact(xsub(cs.rx, rs.rx), xsub(cs.ry, rs.ry), xsub(cs.rz, rs.rz), xsub(cs.vx, rs.vx),
+                                      xsub(cs.vy, rs.vy), xsub(cs.vz, rs.vz), a.dt, a.threshold_km, a.vmin2);
+    if (res == FILTER_CO_ORBITING) ++co;
+    if (res != FILTER_REFINE) return;
+    const unsigned long long pos = atomicAdd(&a.ctrl->refined, 1ull);
+    if (pos < static_cast<unsigned long long>(surv_cap)) surv[pos] = make_int2(min(ro, c), max(ro, c));
+}
+
+// Bits key - 1, key, key + 1 (bits 0, 1, 2 of the result).
+__device__ __forceinline__ unsigned occ_three(const CountArgs& f, unsigned long long key) {
+    const unsigned long long w = __ldcg(f.occ + fib_slot(key >> 5, f.shift));
+    return static_cast<unsigned>(w >> ((key & 31) + 15)) & 7u;
+}
+
+constexpr int kCellBlock = 128;  // threads of k_cells: a small population's cells spread over all SMs
+constexpr int kCellWarps = kCellBlock / 32;
+constexpr int kCellBlocksPerSm = 8;
+
+__global__ void __launch_bounds__(kCellBlock, kCellBlocksPerSm) k_cells(StepArgs a, CountArgs f, const double* __restrict__ before,
+                                                  const float4* __restrict__ sorted32, const int* __restrict__ orig,
+                                                  int2* __restrict__ surv, int64_t surv_cap) {
+    Ctrl* ctrl = a.ctrl;
+    if (step_void(ctrl)) return;
+    constexpr int kMost = 32 * 14;                         // a warp's cells with their forward neighbours
+    __shared__ int2 hit_span[kCellWarps][kMost];
+    __shared__ unsigned short hit_tag[kCellWarps][kMost];      // lane of the cell | neighbour << 5 (13: the cell itself)
+    __shared__ GridParams g;
+    if (threadIdx.x == 0) g = ctrl->grid;
+    __syncthreads();
+    const int n = live_n(a);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nc = min(n, static_cast<int>(static_cast<unsigned int>(ctrl->placed)));
+    // Cells per warp: 32 lanes' worth, fewer where that would leave most of
+    // the chip's warps idle and the launch as long as one warp's chain.
+    int per_warp = 32;
+    while (per_warp > 8 && nc < per_warp * kCellWarps * static_cast<int>(gridDim.x)) per_warp >>= 1;
+    if (per_warp * static_cast<int>(blockIdx.x * kCellWarps) >= nc) return;
+    const PairGate pg = pair_gate(a);
+    const int per = f.per;
+    int2* span = hit_span[warp];
+    unsigned short* tag = hit_tag[warp];
+    unsigned long long cand = 0;
+    unsigned int co = 0, full = 0;
+    bool over = false;
+    for (int w0 = per_warp * (blockIdx.x * kCellWarps + warp); w0 < nc; w0 += per_warp * kCellWarps * gridDim.x) {
+        const int c = lane < per_warp ? w0 + lane : nc;
+        unsigned long long key = 0;
+        int2 own = make_int2(0, 0);
+        unsigned hits = 0;  // bit o: forward neighbour o may exist; bit 13: pairs inside the cell
+        if (c < nc) {
+            key = f.cell_key[c];
+            own = f.cell_span[c];
+            const unsigned long long dx = 1ull << (g.w[1] + g.w[2]), dy = 1ull << g.w[2];
+            hits = occ_three(f, key + dx - dy) | (occ_three(f, key + dx) << 3) | (occ_three(f, key + dx + dy) << 6) |
+                   (occ_three(f, key + dy) << 9) | ((occ_three(f, key) >> 2) << 12) | (own.y > 1 ? 1u << 13 : 0u);
+        }
+        int at = __popc(hits);
+        const int mine = at;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += y;
+        }
+        const int total = __shfl_sync(0xffffffffu, at, 31);
+        at -= mine;
+        __syncwarp();
+        for (int e = at; hits; ++e) {
+            const int o = __ffs(hits) - 1;
+            hits &= hits - 1;
+            tag[e] = static_cast<unsigned short>(lane | (o << 5));
+        }
+        __syncwarp();
+        // The warp's lookups spread over its lanes.
+        for (int h = 0; h < total; h += 32) {
+            const int e = h + lane;
+            const unsigned t = e < total ? tag[e] : 0u;
+            const int src = t & 31, o = static_cast<int>(t >> 5);
+            const unsigned long long k = __shfl_sync(0xffffffffu, key, src);
+            const int2 same = make_int2(__shfl_sync(0xffffffffu, own.x, src), __shfl_sync(0xffffffffu, own.y, src));
+            if (e < total) {
+                int2 sp = same;
+                if (o < 13) {
+                    const unsigned long long want = forward_key(g, k, o);
+                    const int s = want != kEmpty ? cell_find(f, want) : -1;
+                    sp = s >= 0 ? f.span[s] : make_int2(0, 0);
+                }
+                span[e] = sp;
+            }
+        }
+        __syncwarp();
+        int other = 0;
+        const int ahead = mine - (own.y > 1 ? 1 : 0);  // entries of neighbours
+        for (int e = at; e < at + ahead; ++e) other += span[e].y;
+        // Candidate pairs of the cell (the pairs the reference visits, src/core/collision.cpp:522-538).
+        const unsigned long long pairs = static_cast<unsigned long long>(own.y) * (own.y > 0 ? own.y - 1 : 0) / 2 +
+                                         static_cast<unsigned long long>(own.y) * other;
+        cand += pairs;
+        const bool tiled = pairs > kLightPairs;
+        // Light cells: their pairs, 32 entries at a time, spread over the lanes.
+        for (int h = 0; h < total; h += 32) {
+            const int e = h + lane;
+            const unsigned tg = e < total ? tag[e] : 0u;
+            const int2 sp = e < total ? span[e] : make_int2(0, 0);
+            const int src = tg & 31;
+            const int eo = static_cast<int>(tg >> 5);
+            const int eb = __shfl_sync(0xffffffffu, own.x, src);
+            const int ek = __shfl_sync(0xffffffffu, own.y, src);
+            const bool skip = __shfl_sync(0xffffffffu, tiled ? 1 : 0, src) != 0;
+            int upto = e >= total || skip ? 0 : (eo < 13 ? ek * sp.y : ek * (ek - 1) / 2);
+            // At most a pair each, as in a sparse population: every lane takes its own.
+            const bool single = __all_sync(0xffffffffu, upto <= 1);
+            const bool mine1 = upto == 1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += y;
+            }
+            const int all = __shfl_sync(0xffffffffu, upto, 31);
+#pragma unroll 1
+            for (int q0 = 0; q0 < (single ? min(all, 1) : all); q0 += 32) {
+                const int q = single ? (mine1 ? upto - 1 : all) : q0 + lane;
+                // The entry of pair q: the first whose inclusive sum exceeds it.
+                int x = single ? lane : 0;
+                if (!single) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const int v = __shfl_sync(0xffffffffu, upto, x + o - 1);
+                        if (v <= q) x += o;
+                    }
+                }
+                const int before_x = __shfl_sync(0xffffffffu, upto, x > 0 ? x - 1 : 0);
+                const int b0 = __shfl_sync(0xffffffffu, eb, x & 31), k = __shfl_sync(0xffffffffu, ek, x & 31);
+                const int o = __shfl_sync(0xffffffffu, eo, x & 31), s0 = __shfl_sync(0xffffffffu, sp.x, x & 31);
+                if (q >= all) continue;
+                int rem = q - (x > 0 ? before_x : 0);
+                int row, col;
+                float4 off = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (o < 13) {
+                    col = rem / k;
+                    row = rem - col * k;
+                    int dx, dy, dz;
+                    forward_offset(o, dx, dy, dz);
+                    off = make_float4(static_cast<float>(dx) * pg.cell, static_cast<float>(dy) * pg.cell,
+                                      static_cast<float>(dz) * pg.cell, 0.f);
+                } else {
+                    col = 1;  // inside the cell: each pair once
+                    while (rem >= col) rem -= col++;
+                    row = rem;
+                }
+                Rec32 cr = ld_rec32(sorted32 + 2 * static_cast<int64_t>(s0 + col));
+                const Rec32 rr = ld_rec32(sorted32 + 2 * static_cast<int64_t>(b0 + row));
+                if (o < 13) {
+                    cr.p.x += off.x;
+                    cr.p.y += off.y;
+                    cr.p.z += off.z;
+                }
+                light_pair(a, pg, cr, rr, s0 + col, b0 + row, before, orig, surv, surv_cap, co, full);
+            }
+        }
+        const unsigned tm = __ballot_sync(0xffffffffu, tiled);
+        if (!tm) continue;
+        // Column tables and work items of the others. Items of heavy cells
+        // from the front of the list, the rest from its back: the pair kernel
+        // takes the front ones first.
+        const int L = own.y + other, ta = (own.y + 31) >> 5, tc = (L + 31) >> 5;
+        const bool heavy = heavy_cell(own.y, L);
+        const unsigned int n_items = tiled ? cell_items(ta, tc, per) : 0u;
+        unsigned int front = heavy ? n_items : 0u, back = heavy ? 0u : n_items;
+        const unsigned int f0 = front, k0 = back;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int x = __shfl_up_sync(0xffffffffu, front, o), y = __shfl_up_sync(0xffffffffu, back, o);
+            if (lane >= o) {
+                front += x;
+                back += y;
+            }
+        }
+        unsigned int fb = 0, kb = 0, tb = 0;
+        if (lane == 31) {
+            fb = front ? atomicAdd(&ctrl->n_items, front) : 0u;
+            kb = back ? atomicAdd(&ctrl->n_items_back, back) : 0u;
+            tb = atomicAdd(&ctrl->n_tabs, static_cast<unsigned int>(__popc(tm)));
+        }
+        fb = __shfl_sync(0xffffffffu, fb, 31);
+        kb = __shfl_sync(0xffffffffu, kb, 31);
+        tb = __shfl_sync(0xffffffffu, tb, 31);
+        const int64_t base = heavy ? static_cast<int64_t>(fb) + front - f0 : static_cast<int64_t>(kb) + back - k0;
+        const int t = static_cast<int>(tb) + __popc(tm & lanemask_lt());
+        if (tiled) {
+            int2* table = f.col_tab + 16 * static_cast<int64_t>(t);
+            table[0] = make_int2(0, own.x);
+            unsigned long long ids = 0;
+            int nseg = 1, start = own.y;
+            for (int e = at; e < at + ahead; ++e) {
+                const int2 sp = span[e];
+                if (sp.y <= 0) continue;
+                table[nseg] = make_int2(start, sp.x);
+                ids |= static_cast<unsigned long long>((tag[e] >> 5) + 1) << (4 * nseg);
+                ++nseg;
+                start += sp.y;
+            }
+            table[14] = make_int2(static_cast<int>(static_cast<unsigned int>(ids)),
+                                  static_cast<int>(static_cast<unsigned int>(ids >> 32)));
+            table[15] = make_int2(start, nseg);
+        }
+        const bool small = tiled && n_items <= 32;
+        if (small) {
+            int64_t w = base;
+            for (int ra = 0; ra < ta; ++ra)
+                for (int cb = ra; cb < tc; cb += per, ++w) {
+                    if (w < f.items_cap)
+                        f.items[heavy ? w : f.items_cap - 1 - w] = work_item(t, ra, cb, min(per, tc - cb), own.x);
+                    else
+                        over = true;
+                }
+        }
+        // Cells with more than 32 items (all heavy): the warp writes them together.
+        unsigned big = __ballot_sync(0xffffffffu, tiled && !small);
+        while (big) {
+            const int src = __ffs(big) - 1;
+            big &= big - 1;
+            const int tt = __shfl_sync(0xffffffffu, t, src), sa = __shfl_sync(0xffffffffu, ta, src),
+                      sc = __shfl_sync(0xffffffffu, tc, src), bb = __shfl_sync(0xffffffffu, own.x, src);
+            int64_t wbase = __shfl_sync(0xffffffffu, base, src);
+            for (int a0 = 0; a0 < sa; a0 += 32) {
+                const int ra = a0 + lane;
+                const unsigned int some = ra < sa ? row_block_items(ra, sc, per) : 0u;
+                unsigned int upto = some;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned int y = __shfl_up_sync(0xffffffffu, upto, o);
+                    if (lane >= o) upto += y;
+                }
+                int64_t w = wbase + (upto - some);
+                for (int cb = ra; ra < sa && cb < sc; cb += per, ++w) {
+                    if (w < f.items_cap) f.items[w] = work_item(tt, ra, cb, min(per, sc - cb), bb);
+                    else over = true;
+                }
+                wbase += __shfl_sync(0xffffffffu, upto, 31);
+            }
+        }
+    }
+    if (over) atomicOr(&ctrl->flags, FLAG_ITEMS_OVERFLOW);
+    cand = warp_sum(cand);
+    co = warp_sum(co);
+    full = warp_sum(full);
+    if (lane == 0) {
+        if (cand) atomicAdd(&ctrl->candidates, cand);
+        if (co) atomicAdd(&ctrl->co_orbiting, static_cast<unsigned long long>(co));
+        if (full) atomicAdd(&ctrl->exact_evals, static_cast<unsigned long long>(full));
+    }
+}
+
+
 // Blocks of the fused kernel per device (0: not available), set up on first use.
 std::atomic<int> g_fused_grid[kMaxSmDevices];
 
@@ -3444,6 +4032,51 @@ void launch_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream
                                                            b.items_cap, a.tune.item_col_blocks);
 }
 
+// The counted cell build: packed keys, FP32-gated pair kernels.
+bool cells_counted(const DeviceBuffers& b, const StepArgs& a) {
+    return a.tune.sort_fused == 2 && b.place && a.pack_bits > 0 && a.n > 0 && f32_records(a);
+}
+
+namespace {
+// Hash slots of a step's counted build: a power of two above 5/4 of the
+// objects (above 5/2 up to a million: the smaller tables stay in L2 at that
+// size, and a half as crowded one loses fewer exchanges), at most the whole table.
+int64_t count_slots(const DeviceBuffers& b, int n) {
+    const int64_t want = n <= (1 << 20) ? 5 * static_cast<int64_t>(n) / 2 : 5 * static_cast<int64_t>(n) / 4;
+    int64_t slots = 64;
+    while (slots < b.hash_cap && slots < want) slots <<= 1;
+    return slots;
+}
+}  // namespace
+
+void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, cudaStream_t stream) {
+    CountArgs f{};
+    f.keys = b.keys[0];
+    f.hk = b.hash_keys;
+    f.slots = static_cast<unsigned long long>(count_slots(b, a.n));
+    f.occ = b.occ;
+    f.shift = 64;
+    for (unsigned long long q = f.slots / 4; q > 1; q >>= 1) --f.shift;
+    f.cbits = a.pack_bits + 1;  // a count of all n objects needs one bit more than an index
+    f.place = b.place;
+    f.span = b.span;
+    f.cell_key = b.cell_key;
+    f.cell_span = b.cell_span;
+    f.sorted_orig = b.sorted_orig;
+    f.sorted32 = b.sorted32;
+    f.rec32 = b.rec32;
+    f.col_tab = b.col_tab;
+    f.items = b.items;
+    f.items_cap = b.items_cap;
+    f.per = a.tune.item_col_blocks;
+    if (screen) k_place<true><<<grid_for(a.n, 8), kBlock, 0, stream>>>(a, f, b.state[a.src], b.alive[1 - a.src]);
+    else k_place<false><<<grid_for(a.n, 8), kBlock, 0, stream>>>(a, f, b.state[a.src], b.alive[1 - a.src]);
+    k_number<<<grid_for(static_cast<int64_t>(f.slots / 4), 6), kBlock, 0, stream>>>(a, f);
+    k_scatter<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a, f);
+    k_cells<<<grid_for_block(4 * static_cast<int64_t>(a.n), kCellBlocksPerSm, kCellBlock), kCellBlock, 0, stream>>>(
+        a, f, b.state[a.src], b.sorted32, b.sorted_orig, b.survivors, b.surv_cap);
+}
+
 void launch_pairs(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
     // Default: the resident block count of each kernel.
     if (f32_records(a)) {
@@ -3477,7 +4110,8 @@ void launch_pairs(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream
 void launch_refine(const DeviceBuffers& b, const StepArgs& a, ks_conjunction* conj_out, int64_t conj_cap,
                    ChunkCtrl* chunk, cudaStream_t stream) {
     k_refine_exact<<<sm_count() * 2, kBlock, 0, stream>>>(a, b.state[a.src], b.state[1 - a.src], b.size_m,
-                                                         b.survivors, b.surv_cap, conj_out, conj_cap, chunk);
+                                                         b.survivors, b.surv_cap, conj_out, conj_cap, chunk,
+                                                         b.hash_keys, b.occ, cells_counted(b, a) ? count_slots(b, a.n) : 0);
 }
 
 cudaError_t measure_fp64(double* addmul_per_s, double* fma_per_s, cudaStream_t stream) {

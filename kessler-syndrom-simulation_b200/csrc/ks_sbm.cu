@@ -598,7 +598,7 @@ __global__ void k_step_gate(Ctrl* ctrl, int step_in_chunk, int steps_in_chunk, C
     const bool void_step = (f & (FLAG_TIMEOUT | FLAG_SORT_BITS | FLAG_KEY_RANGE | FLAG_PACK_WIDTH |
                                  FLAG_COLL_OVERFLOW | FLAG_ITEMS_OVERFLOW)) != 0 ||
                            ctrl->refined > static_cast<unsigned long long>(surv_cap) ||
-                           static_cast<int64_t>(ctrl->n_items) > items_cap || (chunk->flags & FLAG_CONJ_OVERFLOW) != 0;
+                           items_total(*ctrl) > items_cap || (chunk->flags & FLAG_CONJ_OVERFLOW) != 0;
     if (!void_step) return;
     chunk->halt_step = step_in_chunk;
     Ctrl* first = ctrl - step_in_chunk;
