@@ -258,7 +258,7 @@ class Engine:
         a = _states(after, n)
         al = np.ascontiguousarray(alive_after, dtype=np.uint8)
         sz = np.ascontiguousarray(size_m, dtype=np.float64)
-        cap = 1024
+        cap = max(1024, n)  # untouched rows cost nothing; a short buffer costs a second screening
         while True:
             out = np.zeros(cap, dtype=CONJ_DTYPE)
             stats = np.zeros(1, dtype=STATS_DTYPE)

@@ -36,6 +36,10 @@ namespace {
 
 constexpr int kPhases = 7;  // event slots per step: 0..5 the phases, 6 before the step's L2 flush
 constexpr int kMaxReplays = 6;
+// One-shot screening: end states and sizes up to this many bytes go up with
+// the start states (a plain copy of 1 MB takes about 100 us); beyond, one more
+// round trip and a gather of the pairs' rows take less.
+constexpr size_t kLateBytes = size_t(1) << 20;
 constexpr int64_t kSbmChunkEvents = 65536;  // breakup records one chunk holds (device fragmentation)
 
 }  // namespace
@@ -91,6 +95,23 @@ struct ks_ctx {
     std::vector<int64_t> offsets;  // realisation offsets (batches)
     void* l2_flush = nullptr;
     int64_t l2_flush_bytes = 0;
+
+    // One-shot screening: end states and sizes of the pairs to refine, gathered
+    // on the host, and the pairs (pinned).
+    double* h_rows = nullptr;
+    int2* h_pairs = nullptr;
+    double* d_rows = nullptr;
+    int64_t rows_cap = 0;
+
+    // Runs without screening: two slots of step parameters and loss counts, so
+    // that the host prepares one chunk while the device runs another.
+    struct Plain {
+        StepParams* h_params = nullptr;   // 2 x kManySteps
+        StepParams* d_params = nullptr;
+        unsigned int* h_counts = nullptr;  // 2 x (1 + kManySteps): alive at the start, lost in each step
+        unsigned int* d_counts = nullptr;
+        cudaEvent_t done[2] = {nullptr, nullptr};
+    } plain;
 
     // Fragmentation on the device (ks_set_breakup_mode KS_BREAKUP_DEVICE):
     // the population grows inside chunks up to dev_cap objects; no replays,
@@ -149,7 +170,7 @@ void free_objects(ks_ctx* ctx) {
     dfree(b.size_m); dfree(b.real_id); dfree(b.ckpt_state); dfree(b.ckpt_alive); dfree(b.block_counts);
     dfree(b.sort_hist); dfree(b.sort_status); dfree(b.sort_ctr);
     dfree(b.cell_begin); dfree(b.cell_key); dfree(b.nbr); dfree(b.cell_len); dfree(b.col_tab); dfree(b.item_part); dfree(b.hash_keys); dfree(b.hash_vals);
-    dfree(b.place); dfree(b.span); dfree(b.cell_span); dfree(b.occ);
+    dfree(b.occ);
     dfree(b.sorted); dfree(b.sorted32); dfree(b.rec32); dfree(b.sorted_orig); dfree(b.fused);
     b.fused_grid = 0;
     dfree(b.n_live); dfree(b.mass_kg); dfree(b.a2m); dfree(b.event_of); dfree(b.coll); dfree(b.sbm_work);
@@ -200,9 +221,6 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     b.hash_cap = h;
     KS_CUDA(cudaMalloc(&b.hash_keys, sizeof(unsigned long long) * h));
     KS_CUDA(cudaMalloc(&b.hash_vals, sizeof(int) * h));
-    KS_CUDA(cudaMalloc(&b.place, sizeof(int2) * cap));
-    KS_CUDA(cudaMalloc(&b.span, sizeof(int2) * h));
-    KS_CUDA(cudaMalloc(&b.cell_span, sizeof(int2) * cap));
     KS_CUDA(cudaMalloc(&b.occ, sizeof(unsigned long long) * (h / 4)));
     KS_CUDA(cudaMemset(b.occ, 0, sizeof(unsigned long long) * (h / 4)));
     KS_CUDA(cudaMalloc(&b.sorted, sizeof(double) * 6 * cap));
@@ -385,16 +403,28 @@ int estimate_bits(const Ctrl& c, double dt, double thr, int sub, int rbits, doub
     return bits + 3 * sub;
 }
 
-void fill_params(ks_ctx* ctx, int k_steps, double t_start, int64_t step0, double* t_end) {
+void fill_steps(const ks_ctx* ctx, StepParams* rows, int k_steps, double t_start, int64_t step0, double* t_end) {
     double t = t_start;
     for (int k = 0; k < k_steps; ++k) {
-        StepParams& sp = ctx->h_params[k];
+        StepParams& sp = rows[k];
         sp.t0 = t;
         sp.step = step0 + k;
-        ks::moon_stages(ctx->epoch_jd, t, ctx->dt, sp.m);
+        if (k == 0) {
+            ks::moon_stages(ctx->epoch_jd, t, ctx->dt, sp.m);
+        } else {
+            // A step starts at the instant the one before it ended: the same
+            // Julian date, the same lunar stage.
+            sp.m[0] = rows[k - 1].m[2];
+            ks::moon_stage_at(ctx->epoch_jd + (t + ctx->dt / 2) / 86400.0, sp.m[1]);
+            ks::moon_stage_at(ctx->epoch_jd + (t + ctx->dt) / 86400.0, sp.m[2]);
+        }
         t += ctx->dt;  // Simulation::step (src/core/orbital.cpp:299)
     }
     *t_end = t;
+}
+
+void fill_params(ks_ctx* ctx, int k_steps, double t_start, int64_t step0, double* t_end) {
+    fill_steps(ctx, ctx->h_params, k_steps, t_start, step0, t_end);
 }
 
 // Bits that hold every object index 0 .. n-1 (at least 1).
@@ -437,6 +467,9 @@ StepArgs step_args(ks_ctx* ctx, int k, int k_steps, int src) {
         a.coll_cap = ctx->b.coll_cap;
         a.pack_bits = ctx->pack_keys ? index_bits(ctx->b.cap) : 0;
     }
+    // Kernels of a step start while their predecessors drain, unless events
+    // or flushes lie between them.
+    a.overlap = ctx->profiling == 0 && ctx->l2_flush_bytes == 0;
     // The fused sort counts its own digits: the propagation need not.
     if (a.hist && (ks::cells_counted(ctx->b, a) || ks::sort_cells_fused(ctx->b, a))) a.hist = nullptr;
     return a;
@@ -976,6 +1009,103 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
     return KS_OK;
 }
 
+void free_plain(ks_ctx* ctx) {
+    ks_ctx::Plain& p = ctx->plain;
+    if (p.h_params) cudaFreeHost(p.h_params);
+    if (p.h_counts) cudaFreeHost(p.h_counts);
+    dfree(p.d_params);
+    dfree(p.d_counts);
+    for (cudaEvent_t& e : p.done) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
+    p.h_params = nullptr;
+    p.h_counts = nullptr;
+}
+
+int ensure_plain(ks_ctx* ctx) {
+    ks_ctx::Plain& p = ctx->plain;
+    if (p.done[1]) return KS_OK;
+    free_plain(ctx);
+    KS_CUDA(cudaHostAlloc(&p.h_params, sizeof(StepParams) * 2 * ks::kManySteps, cudaHostAllocDefault));
+    KS_CUDA(cudaHostAlloc(&p.h_counts, sizeof(unsigned int) * 2 * (1 + ks::kManySteps), cudaHostAllocDefault));
+    KS_CUDA(cudaMalloc(&p.d_params, sizeof(StepParams) * 2 * ks::kManySteps));
+    KS_CUDA(cudaMalloc(&p.d_counts, sizeof(unsigned int) * 2 * (1 + ks::kManySteps)));
+    for (cudaEvent_t& e : p.done) KS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return KS_OK;
+}
+
+// Steps without screening: nothing of a step is needed before the next one,
+// so a launch carries kManySteps of them, and the next chunk's lunar rows are
+// prepared while it runs. (With per-phase timing or the L2 flush before every
+// step, steps are launched one by one.)
+bool plain_run(const ks_ctx* ctx) {
+    return !ctx->screening && !ctx->dev_sbm && !ctx->profiling && ctx->l2_flush_bytes == 0 && ctx->n > 0;
+}
+
+int run_plain(ks_ctx* ctx, int64_t steps) {
+    const HostClock::time_point h0 = HostClock::now();
+    int rc = ensure_plain(ctx);
+    if (rc) return rc;
+    ks_ctx::Plain& p = ctx->plain;
+    ks::DeviceBuffers& b = ctx->b;
+    constexpr int kCounts = 1 + ks::kManySteps;
+    int64_t pending[2] = {0, 0}, first[2] = {0, 0};
+    auto collect = [&](int slot) -> int {
+        if (pending[slot] == 0) return KS_OK;
+        const HostClock::time_point hs = HostClock::now();
+        KS_CUDA(cudaEventSynchronize(p.done[slot]));
+        ctx->timing.host_sync_ms += host_ms(hs, HostClock::now());
+        const unsigned int* counts = p.h_counts + slot * kCounts;
+        int64_t alive = counts[0];
+        for (int64_t k = 0; k < pending[slot]; ++k) {
+            ctx->timing.object_steps += alive;
+            alive -= counts[1 + k];
+            ks_step_stats st{};
+            st.step = first[slot] + k;
+            st.alive = static_cast<int32_t>(alive);
+            ctx->stats_out.push_back(st);
+        }
+        ctx->timing.steps += pending[slot];
+        pending[slot] = 0;
+        return KS_OK;
+    };
+    int slot = 0;
+    for (int64_t left = steps; left > 0; slot ^= 1) {
+        if ((rc = collect(slot))) return rc;
+        const int k = static_cast<int>(std::min<int64_t>(left, ks::kManySteps));
+        StepParams* rows = p.h_params + slot * ks::kManySteps;
+        double t_end = 0.0;
+        const HostClock::time_point hp = HostClock::now();
+        fill_steps(ctx, rows, k, ctx->t, ctx->steps_done, &t_end);
+        const HostClock::time_point hl = HostClock::now();
+        ctx->timing.host_prep_ms += host_ms(hp, hl);
+        StepParams* d_rows = p.d_params + slot * ks::kManySteps;
+        unsigned int* d_counts = p.d_counts + slot * kCounts;
+        KS_CUDA(cudaMemcpyAsync(d_rows, rows, sizeof(StepParams) * k, cudaMemcpyHostToDevice, ctx->stream));
+        KS_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(unsigned int) * kCounts, ctx->stream));
+        const int dst = ctx->cur ^ (k & 1);
+        ks::launch_propagate_steps(force_consts(), ctx->dt, ctx->precision, static_cast<int>(ctx->n), k, d_rows,
+                                   b.state[ctx->cur], b.state[dst], b.alive[ctx->cur], b.alive[dst], d_counts,
+                                   d_counts + 1, ctx->stream);
+        KS_CUDA(cudaGetLastError());
+        KS_CUDA(cudaMemcpyAsync(p.h_counts + slot * kCounts, d_counts, sizeof(unsigned int) * kCounts,
+                                cudaMemcpyDeviceToHost, ctx->stream));
+        KS_CUDA(cudaEventRecord(p.done[slot], ctx->stream));
+        ctx->timing.host_launch_ms += host_ms(hl, HostClock::now());
+        first[slot] = ctx->steps_done;
+        pending[slot] = k;
+        ctx->cur = dst;
+        ctx->steps_done += k;
+        ctx->t = t_end;
+        left -= k;
+    }
+    for (int q = 0; q < 2; ++q, slot ^= 1)
+        if ((rc = collect(slot))) return rc;
+    ctx->timing.host_chunk_ms += host_ms(h0, HostClock::now());
+    return KS_OK;
+}
+
 int seed_speculation(ks_ctx* ctx) {
     ks::launch_seed_ctrl(ctx->b, static_cast<int>(ctx->n), ctx->cur, carry_slot(ctx), 1, ctx->stream);
     Ctrl c{};
@@ -990,6 +1120,23 @@ int seed_speculation(ks_ctx* ctx) {
     if (passes != ctx->sort_passes || pack != ctx->pack_keys) drop_graphs(ctx);
     ctx->sort_passes = passes;
     ctx->pack_keys = pack;
+    return KS_OK;
+}
+
+// Room for the ends of np pairs (12 + 2 doubles each) and for the pairs.
+int ensure_rows(ks_ctx* ctx, int64_t np) {
+    if (np <= ctx->rows_cap) return KS_OK;
+    np = std::max<int64_t>(np + np / 2, 4096);
+    if (ctx->h_rows) cudaFreeHost(ctx->h_rows);
+    if (ctx->h_pairs) cudaFreeHost(ctx->h_pairs);
+    ctx->h_rows = nullptr;
+    ctx->h_pairs = nullptr;
+    dfree(ctx->d_rows);
+    ctx->rows_cap = 0;
+    KS_CUDA(cudaHostAlloc(&ctx->h_rows, sizeof(double) * 14 * np, cudaHostAllocDefault));
+    KS_CUDA(cudaHostAlloc(&ctx->h_pairs, sizeof(int2) * np, cudaHostAllocDefault));
+    KS_CUDA(cudaMalloc(&ctx->d_rows, sizeof(double) * 14 * np));
+    ctx->rows_cap = np;
     return KS_OK;
 }
 
@@ -1376,6 +1523,9 @@ void ks_destroy(ks_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    if (ctx->h_rows) cudaFreeHost(ctx->h_rows);
+    if (ctx->h_pairs) cudaFreeHost(ctx->h_pairs);
+    dfree(ctx->d_rows);
     drop_graphs(ctx);
     free_objects(ctx);
     if (ctx->l2_flush) cudaFree(ctx->l2_flush);
@@ -1383,6 +1533,7 @@ void ks_destroy(ks_ctx* ctx) {
     dfree(ctx->b.items);
     if (ctx->frag_scratch) cudaFree(ctx->frag_scratch);
     free_conj(ctx);
+    free_plain(ctx);
     dfree(ctx->b.ctrl);
     dfree(ctx->b.chunk);
     dfree(ctx->b.params);
@@ -1802,6 +1953,7 @@ int ks_run(ks_ctx* ctx, int64_t steps) {
     if (!ctx->has_pop) return fail(ctx, KS_ERR_STATE, "ks_run: no population");
     cudaSetDevice(ctx->device);
     ctx->timing = ks_timing{};
+    if (plain_run(ctx)) return run_plain(ctx, steps);
     const int chunk = ctx->steps_per_graph > 0 ? ctx->steps_per_graph : 64;
     int rc = ensure_chunk(ctx, chunk);
     if (rc) return rc;
@@ -1823,7 +1975,7 @@ int ks_prepare_run(ks_ctx* ctx) {
     if (!ctx) return KS_ERR_ARG;
     if (!ctx->has_pop) return fail(ctx, KS_ERR_STATE, "ks_prepare_run: no population");
     cudaSetDevice(ctx->device);
-    if (ctx->steps_per_graph <= 0 || ctx->dev_sbm) return KS_OK;
+    if (ctx->steps_per_graph <= 0 || ctx->dev_sbm || plain_run(ctx)) return KS_OK;
     const int k = ctx->steps_per_graph;
     int rc = ensure_chunk(ctx, k);
     if (!rc) rc = plan_chunk(ctx, k);
@@ -2259,9 +2411,21 @@ int ks_screen(ks_ctx* ctx, int64_t n, const double* before, const double* after,
     ctx->rbits = 0;
     ctx->offsets.assign({0, n});
     reset_breakup_run(ctx);
-    rc = upload_population(ctx, n, before, size_m, nullptr, 0);
-    if (!rc) rc = upload_population(ctx, n, after, nullptr, alive_after, 1);
-    if (rc) return rc;
+    // The kernels before the refinement read the start states and the flags
+    // alone. The end states and sizes of a larger population are not sent: the
+    // refinement gets those of its pairs, gathered here once the pairs are known.
+    const size_t rows = static_cast<size_t>(n);
+    const bool late = sizeof(double) * 7 * rows >= kLateBytes;
+    KS_CUDA(cudaMemcpyAsync(ctx->b.state[0], before, sizeof(double) * 6 * rows, cudaMemcpyHostToDevice, ctx->stream));
+    KS_CUDA(cudaMemcpyAsync(ctx->b.alive[1], alive_after, rows, cudaMemcpyHostToDevice, ctx->stream));
+    bool sent = !late;
+    auto send_ends = [&]() -> int {
+        KS_CUDA(cudaMemcpyAsync(ctx->b.state[1], after, sizeof(double) * 6 * rows, cudaMemcpyHostToDevice, ctx->stream));
+        KS_CUDA(cudaMemcpyAsync(ctx->b.size_m, size_m, sizeof(double) * rows, cudaMemcpyHostToDevice, ctx->stream));
+        sent = true;
+        return KS_OK;
+    };
+    if (!late && (rc = send_ends())) return rc;
     const double saved_dt = ctx->dt;
     ctx->dt = dt;
     StepParams sp{};
@@ -2271,20 +2435,77 @@ int ks_screen(ks_ctx* ctx, int64_t n, const double* before, const double* after,
     KS_CUDA(cudaMemcpyAsync(ctx->b.params, ctx->h_params, sizeof(StepParams), cudaMemcpyHostToDevice, ctx->stream));
     std::vector<ks_conjunction> found;
     ks_step_stats st{};
+    bool wide = false;  // keys too wide for the counted build
+    // Records copied back with the control blocks: a call that finds no more takes one round trip.
+    const int64_t with_ctrl = std::min<int64_t>(ctx->b.conj_cap, 512);
+    stash_pending(ctx);
     for (int attempt = 0;; ++attempt) {
-        ks::launch_chunk_init(ctx->b, 1, ctx->stream);
+        ks::launch_screen_init(ctx->b, static_cast<int>(n), ctx->stream);
         StepArgs a = step_args(ctx, 0, 1, 0);
-        a.hist = nullptr;  // keys come from k_screen_keys: the sort counts their digits itself
-        a.pack_bits = 0;
-        ks::launch_seed_ctrl(ctx->b, static_cast<int>(n), 0, a.ctrl, 0, ctx->stream);
-        ks::launch_screen_keys(ctx->b, a, ctx->stream);
-        ks::launch_sort(ctx->b, a, ctx->stream);
-        ks::launch_cells(ctx->b, a, ctx->stream);
+        a.hist = nullptr;  // keys come from the states: a sort counts their digits itself
+        // The counted build keeps a cell's key and count in one word: room for
+        // both is known only once the grid is (FLAG_PACK_WIDTH below).
+        a.pack_bits = ctx->allow_pack && !wide ? index_bits(n) : 0;
+        if (ks::cells_counted(ctx->b, a)) {
+            ks::launch_count_cells(ctx->b, a, true, ctx->stream);
+        } else {
+            a.pack_bits = 0;
+            ks::launch_screen_keys(ctx->b, a, ctx->stream);
+            ks::launch_sort(ctx->b, a, ctx->stream);
+            ks::launch_cells(ctx->b, a, ctx->stream);
+        }
         ks::launch_pairs(ctx->b, a, ctx->stream);
-        ks::launch_refine(ctx->b, a, ctx->b.conj, ctx->b.conj_cap, ctx->b.chunk, ctx->stream);
+        KS_CUDA(cudaGetLastError());
+        bool pairs_fit = true;
+        if (late) {
+            // The pairs, with the control block; then their ends, or the whole arrays where the pairs name most objects.
+            constexpr int64_t kWith = 4096;
+            if ((rc = ensure_rows(ctx, kWith))) { ctx->dt = saved_dt; return rc; }
+            const int64_t with = std::min<int64_t>(kWith, ctx->b.surv_cap);
+            KS_CUDA(cudaMemcpyAsync(ctx->h_ctrl, ctx->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, ctx->stream));
+            KS_CUDA(cudaMemcpyAsync(ctx->h_pairs, ctx->b.survivors, sizeof(int2) * with, cudaMemcpyDeviceToHost, ctx->stream));
+            KS_CUDA(cudaStreamSynchronize(ctx->stream));
+            const Ctrl& c = ctx->h_ctrl[0];
+            // A step that will be repeated or refused is not refined (its lists may hold anything).
+            pairs_fit = c.refined <= static_cast<unsigned long long>(ctx->b.surv_cap) && ks::items_total(c) <= ctx->b.items_cap &&
+                        !(c.flags & (ks::FLAG_KEY_RANGE | ks::FLAG_TIMEOUT | ks::FLAG_SORT_BITS | ks::FLAG_PACK_WIDTH | ks::FLAG_ITEMS_OVERFLOW));
+            const int64_t np = pairs_fit ? static_cast<int64_t>(c.refined) : 0;
+            if (pairs_fit && !sent && 4 * np > n) {
+                if ((rc = send_ends())) { ctx->dt = saved_dt; return rc; }
+            } else if (np > 0 && !sent) {
+                const bool again = np > with || np > ctx->rows_cap;  // more than came along, or the buffer is made anew
+                if ((rc = ensure_rows(ctx, np))) { ctx->dt = saved_dt; return rc; }
+                if (again)
+                    KS_CUDA(cudaMemcpyAsync(ctx->h_pairs, ctx->b.survivors, sizeof(int2) * np, cudaMemcpyDeviceToHost, ctx->stream));
+                KS_CUDA(cudaStreamSynchronize(ctx->stream));
+                double* ends = ctx->h_rows;
+                double* sizes = ctx->h_rows + 12 * np;
+                for (int64_t q = 0; q < np; ++q) {
+                    const int2 p = ctx->h_pairs[q];
+                    std::memcpy(ends + 12 * q, after + 6 * static_cast<int64_t>(p.x), sizeof(double) * 6);
+                    std::memcpy(ends + 12 * q + 6, after + 6 * static_cast<int64_t>(p.y), sizeof(double) * 6);
+                    sizes[2 * q] = size_m[p.x];
+                    sizes[2 * q + 1] = size_m[p.y];
+                }
+                KS_CUDA(cudaMemcpyAsync(ctx->d_rows, ctx->h_rows, sizeof(double) * 14 * np, cudaMemcpyHostToDevice, ctx->stream));
+            }
+            a.overlap = 0;
+        }
+        if (pairs_fit) {
+            const int64_t np = static_cast<int64_t>(ctx->h_ctrl[0].refined);
+            if (!late || sent)
+                ks::launch_refine(ctx->b, a, ctx->b.conj, ctx->b.conj_cap, ctx->b.chunk, ctx->stream);
+            else
+                ks::launch_refine_rows(ctx->b, a, ctx->d_rows, ctx->d_rows + 12 * np, ctx->b.conj, ctx->b.conj_cap, ctx->b.chunk,
+                                       ctx->stream);
+        } else {
+            ks::launch_clear_cells(ctx->b, a, ctx->stream);
+        }
         KS_CUDA(cudaGetLastError());
         KS_CUDA(cudaMemcpyAsync(ctx->h_ctrl, ctx->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, ctx->stream));
         KS_CUDA(cudaMemcpyAsync(ctx->h_chunk, ctx->b.chunk, sizeof(ks::ChunkCtrl), cudaMemcpyDeviceToHost, ctx->stream));
+        if (with_ctrl > 0)
+            KS_CUDA(cudaMemcpyAsync(ctx->h_conj, ctx->b.conj, sizeof(ks_conjunction) * with_ctrl, cudaMemcpyDeviceToHost, ctx->stream));
         KS_CUDA(cudaStreamSynchronize(ctx->stream));
         const Ctrl& c = ctx->h_ctrl[0];
         const int flags = c.flags | ctx->h_chunk->flags;
@@ -2292,7 +2513,7 @@ int ks_screen(ks_ctx* ctx, int64_t n, const double* before, const double* after,
         const bool items_over = ks::items_total(c) > ctx->b.items_cap;
         if (flags & ks::FLAG_KEY_RANGE) { ctx->dt = saved_dt; return fail(ctx, KS_ERR_RANGE, "cell key outside its grid bounds or wider than 63 bits"); }
         if (flags & ks::FLAG_TIMEOUT) { ctx->dt = saved_dt; return fail(ctx, KS_ERR_TIMEOUT, "radix sort look-back or grid barrier wait gave up"); }
-        if (!(flags & (ks::FLAG_CONJ_OVERFLOW | ks::FLAG_SORT_BITS)) && !surv_over && !items_over) {
+        if (!(flags & (ks::FLAG_CONJ_OVERFLOW | ks::FLAG_SORT_BITS | ks::FLAG_PACK_WIDTH)) && !surv_over && !items_over) {
             st.step = 0;
             st.candidate_pairs = static_cast<int64_t>(c.candidates);
             st.refined_pairs = static_cast<int64_t>(c.refined);
@@ -2304,6 +2525,7 @@ int ks_screen(ks_ctx* ctx, int64_t n, const double* before, const double* after,
             break;
         }
         if (attempt >= kMaxReplays) { ctx->dt = saved_dt; return fail(ctx, KS_ERR_OVERFLOW, "ks_screen: buffers overflow"); }
+        if (flags & ks::FLAG_PACK_WIDTH) wide = true;
         if (flags & ks::FLAG_SORT_BITS) ctx->sort_passes = std::max(ctx->sort_passes, passes_for_bits(c.grid.bits));
         if (surv_over && (rc = ensure_survivors(ctx, static_cast<int64_t>(c.refined) * 2))) { ctx->dt = saved_dt; return rc; }
         if (items_over && (rc = ensure_items(ctx, ks::items_total(c) * 3 / 2 + 1024))) { ctx->dt = saved_dt; return rc; }
@@ -2314,10 +2536,11 @@ int ks_screen(ks_ctx* ctx, int64_t n, const double* before, const double* after,
     }
     ctx->dt = saved_dt;
     const int64_t nc = static_cast<int64_t>(ctx->h_chunk->conj_count);
-    stash_pending(ctx);
     if (nc > 0) {
-        KS_CUDA(cudaMemcpyAsync(ctx->h_conj, ctx->b.conj, sizeof(ks_conjunction) * nc, cudaMemcpyDeviceToHost, ctx->stream));
-        KS_CUDA(cudaStreamSynchronize(ctx->stream));
+        if (nc > with_ctrl) {
+            KS_CUDA(cudaMemcpyAsync(ctx->h_conj, ctx->b.conj, sizeof(ks_conjunction) * nc, cudaMemcpyDeviceToHost, ctx->stream));
+            KS_CUDA(cudaStreamSynchronize(ctx->stream));
+        }
         found.assign(ctx->h_conj, ctx->h_conj + nc);
         std::sort(found.begin(), found.end(), conj_less);
     }

@@ -142,11 +142,12 @@ struct DeviceBuffers {
     unsigned long long* hash_keys = nullptr;
     int* hash_vals = nullptr;
     int64_t hash_cap = 0;                  // power of two
-    // Counted cell build (null in the allocation-free entry point, which sorts).
-    unsigned long long* occ = nullptr;     // occupancy words, a quarter of the hash slots (all zero between steps)
-    int2* place = nullptr;                 // per object: its cell's slot, rank in it
-    int2* cell_span = nullptr;             // per cell: first sorted position and objects
-    int2* span = nullptr;                  // per slot: first sorted position and objects of its cell
+    // Counted cell build: occupancy words, a quarter of the hash slots, all
+    // zero between steps (null in the allocation-free entry point, which
+    // sorts). Its other arrays are those of the sorted builds it does not use:
+    // keys[1] each object's slot and rank, sorted each slot's span (8 bytes a
+    // slot, at most 4 slots an object), nbr each cell's span.
+    unsigned long long* occ = nullptr;
     double* sorted = nullptr;              // 6 per sorted entry
     float4* sorted32 = nullptr;            // FP32 records: cell-relative position, velocity, in cell order
     float4* rec32 = nullptr;               // the same records in object order, written with the keys
@@ -234,6 +235,7 @@ struct StepArgs {
     int src;                   // state buffer holding the start of the step (0 or 1)
     unsigned int* hist;        // radix digit histogram the propagation fills with the keys it emits, or null
     float4* rec32;             // FP32 record of each object, written with its key (object order)
+    int overlap;               // the step's kernels may start while their predecessors drain (launch_after)
     int pack_bits;             // > 0: sort keys carry the object index in their low pack_bits bits
     // Fragmentation on the device (null / 0 otherwise): the live population
     // size (kernels bound their loops by it; n above is then the capacity the
@@ -300,6 +302,15 @@ void launch_chunk_init(const DeviceBuffers& b, int k_steps, cudaStream_t stream,
 void launch_seed_ctrl(const DeviceBuffers& b, int n, int src, Ctrl* target, int use_alive_src,
                       cudaStream_t stream);
 void launch_propagate(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
+// `steps` (at most kManySteps) steps without screening in one launch, from
+// in / alive_in to out / alive_out (which may be the same buffers).
+constexpr int kManySteps = 128;
+void launch_propagate_steps(const ForceConsts& fc, double dt, int precision, int n, int steps, const StepParams* sp,
+                            const double* in, double* out, const uint8_t* alive_in, uint8_t* alive_out,
+                            unsigned int* alive0, unsigned int* died, cudaStream_t stream);
+// Control block of a one-shot screening: reset, then the speed and position
+// bounds of the objects alive after the step at their start-of-step states.
+void launch_screen_init(const DeviceBuffers& b, int n, cudaStream_t stream);
 void launch_screen_keys(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 // Fragments born inside a step: rows [first, first + count) advanced over
 // their events' remaining time (spans[row_span[k]]), then their alive flags set.
@@ -335,6 +346,12 @@ void launch_conj_sort(const DeviceBuffers& b, ChunkCtrl* chunk, const double* t_
                       cudaStream_t stream);
 void launch_refine(const DeviceBuffers& b, const StepArgs& a, ks_conjunction* conj_out, int64_t conj_cap,
                    ChunkCtrl* chunk, cudaStream_t stream);
+
+// The same with the pairs' end states (12 doubles a pair) and sizes (2) in the order of the survivors.
+void launch_refine_rows(const DeviceBuffers& b, const StepArgs& a, const double* ends, const double* sizes,
+                        ks_conjunction* conj_out, int64_t conj_cap, ChunkCtrl* chunk, cudaStream_t stream);
+// Empties the counted build's tables, as the refinement does at its end (a step that is not refined).
+void launch_clear_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 
 // Device SBM (ks_sbm.cu). After a step's refinement: voids the rest of the
 // chunk if the step's buffers overflowed, then fragments the step's
