@@ -194,7 +194,7 @@ struct Tuning {
     int box_min_rows = 4;         // split pairs: block-box pruning for tiles with at least this many rows (0: off)
     double cell_scale = 1.0;      // cell edge = reference edge x this (>= 1; changes only candidate counts)
     int prop_block = 128;         // threads per block of the propagation kernels (32..128, multiple of 32)
-    int item_col_blocks = 16;     // column blocks of 32 per pair work item (1..64)
+    int item_col_blocks = 0;      // column blocks of 32 per pair work item (1..64; 0: by the population, item_blocks)
     int lookback_polls = 1 << 22; // polls of a radix-sort look-back before it gives up (FLAG_TIMEOUT)
     int pair_gate_x2 = 1;         // FP32 pair gate on two rows per instruction (packed f32x2)
     int pair_stage2 = 1;          // second FP32 stage: 0 row by row, 1 compacted when sparse, 2 always compacted
@@ -324,6 +324,7 @@ void launch_clear_alive(uint8_t* alive, const int64_t* idx, int count, cudaStrea
 void launch_fix_keys(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 void launch_sort(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 bool f32_records(const StepArgs& a);
+int item_blocks(const Tuning& t, int64_t n);  // column blocks per work item for n objects
 void launch_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 // Fused sort + cell build: blocks per launch on the current device (0: not
 // available), scratch words for that grid, whether a step takes the fused path.

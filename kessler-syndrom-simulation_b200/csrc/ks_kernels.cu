@@ -3792,6 +3792,19 @@ int fused_digit_bits(const StepArgs& a, int K) {
     return (8 * a.sort_passes + 10) / 11 < a.sort_passes ? 11 : 8;
 }
 
+// Column blocks of a pair work item. An item's length is its warp's chain (a
+// column block is a round of dependent loads), the number of items what a
+// dense cell occupies the chip with: one crowded cell in a catalogue wants
+// short items, a population that fills the chip long ones, whose set-up is
+// paid less often. Tile kernel, us a step, at 2 / 4 / 8 / 16 / 32 blocks: 33 000
+// objects with a fresh cloud of 5 000 37 / 47 / 63 / 105 / 185; 28 340 at dt 60 s
+// 20 / 21 / 23 / 28 / 28; 250 000 141 / 119 / 112 / 115 / 127; a million 304 / 250 / 225 /
+// 222 / 237; four million 1324 / 1072 / 944 / 886 / 867.
+int item_blocks(const Tuning& t, int64_t n) {
+    if (t.item_col_blocks > 0) return t.item_col_blocks;
+    return n < (1 << 16) ? 2 : n < (1 << 17) ? 4 : n < (1 << 19) ? 8 : n < (1 << 22) ? 16 : 32;
+}
+
 void launch_sort_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
     const int grid = fused_grid();
     const int K = fused_keys_per_thread(a.n, grid);
@@ -3816,7 +3829,7 @@ void launch_sort_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t s
     f.col_tab = b.col_tab;
     f.items = b.items;
     f.items_cap = b.items_cap;
-    f.per = a.tune.item_col_blocks;
+    f.per = item_blocks(a.tune, a.n);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kFusedThreads);
@@ -4132,12 +4145,12 @@ void launch_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream
     // Left empty for the fused launches, which take it so.
     cudaMemsetAsync(b.hash_keys, 0xFF, sizeof(unsigned long long) * b.hash_cap, stream);
     k_items_count<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a.ctrl, b.cell_begin, b.nbr, b.cell_len, b.col_tab, b.item_part,
-                                                           a.tune.item_col_blocks);
+                                                           item_blocks(a.tune, a.n));
     // Offsets of the heavy, then the light cells' items per chunk of cells, and their total.
     k_scan_small<<<1, 1024, 0, stream>>>(b.item_part, static_cast<int>(2 * ((b.cap + kBlock - 1) / kBlock)),
                                          &a.ctrl->n_items, &a.ctrl->n_cells, 2);
     k_items_write<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a.ctrl, b.cell_begin, b.cell_len, b.item_part, b.items,
-                                                           b.items_cap, a.tune.item_col_blocks);
+                                                           b.items_cap, item_blocks(a.tune, a.n));
 }
 
 // The counted cell build: packed keys, FP32-gated pair kernels.
@@ -4176,7 +4189,7 @@ void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, 
     f.col_tab = b.col_tab;
     f.items = b.items;
     f.items_cap = b.items_cap;
-    f.per = a.tune.item_col_blocks;
+    f.per = item_blocks(a.tune, a.n);
     const bool o = a.overlap != 0;
     launch_after(o && !screen, screen ? k_place<true> : k_place<false>, grid_for(a.n, 8), kBlock, stream, a, f,
                  b.state[a.src], b.alive[1 - a.src]);

@@ -200,6 +200,7 @@ int screen_noalloc(int64_t n, const double* before, const double* after, const u
     NA_CUDA(cudaMemcpyAsync(b.params, &sp, sizeof(sp), cudaMemcpyHostToDevice, s));
 
     ks::StepArgs a{};
+    a.tune.item_col_blocks = 16;  // the fixed item list is sized for items of this length
     a.fc.neg_mu_earth = -ks::kMuEarth;
     a.fc.k_j2 = ks::j2_numerator();
     a.fc.mu_moon = ks::kMuMoon;
