@@ -89,6 +89,8 @@ struct ks_ctx {
     int64_t chunk_spec = 0;    // records a chunk copies back with its control blocks
     int64_t graph_spec[2] = {0, 0};  // the same, as captured in graph_exec[]
     int64_t graph_n[2] = {-1, -1};   // population size graph_exec[] was captured for
+    int64_t direct_n[2] = {-1, -1};  // population size of a whole chunk launched without a graph since the last one was dropped
+    int64_t launched_spec = 0;       // chunk_spec as the last chunk was launched with
     bool allow_pack = true;    // tuning: packing allowed where the keys leave room
     int realisations = 1;
     int rbits = 0;
@@ -158,6 +160,7 @@ void dfree(T*& p) {
 }
 
 void drop_graphs(ks_ctx* ctx) {
+    ctx->direct_n[0] = ctx->direct_n[1] = -1;
     for (auto& g : ctx->graph_exec) {
         if (g) cudaGraphExecDestroy(g);
         g = nullptr;
@@ -563,8 +566,13 @@ void enqueue_chunk(ks_ctx* ctx, int k_steps, int src0, bool capturing) {
                         cudaMemcpyDeviceToHost, s);
 }
 
-// Captures and instantiates the chunk's graph if it does not exist yet.
-int ensure_graph(ks_ctx* ctx, int k_steps) {
+// Captures and instantiates the chunk's graph if it does not exist yet. The
+// first chunk of a configuration goes without one: its launches are queued
+// while the device works, whereas capturing 32 steps and instantiating their
+// graph takes the host longer (some 2 ms) than running them, which a single
+// chunk - a trial of a breakup study, whose fragments change the population's
+// size - never wins back (a trial of 28 340 objects and 36 steps: about 1.4 of 5.6 ms).
+int ensure_graph(ks_ctx* ctx, int k_steps, bool prepare = false) {
     const bool use_graph = ctx->steps_per_graph > 0 && k_steps == ctx->steps_per_graph;
     if (!use_graph) return KS_OK;
     cudaGraphExec_t& exec = ctx->graph_exec[ctx->cur];
@@ -572,6 +580,11 @@ int ensure_graph(ks_ctx* ctx, int k_steps) {
     // the host; on the device they hold the capacity): a graph captured for
     // another size, as after fragments were appended, is captured again.
     if (exec && !ctx->dev_sbm && ctx->graph_n[ctx->cur] != ctx->n) drop_graphs(ctx);
+    const int64_t size = ctx->dev_sbm ? ctx->b.cap : ctx->n;
+    if (!exec && !prepare && ctx->direct_n[ctx->cur] != size) {
+        ctx->direct_n[ctx->cur] = size;
+        return KS_OK;
+    }
     if (!exec) {
         cudaGraph_t g = nullptr;
         KS_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
@@ -595,15 +608,16 @@ int ensure_graph(ks_ctx* ctx, int k_steps) {
 }
 
 int launch_chunk(ks_ctx* ctx, int k_steps) {
-    const bool use_graph = ctx->steps_per_graph > 0 && k_steps == ctx->steps_per_graph;
-    if (!use_graph) {
-        enqueue_chunk(ctx, k_steps, ctx->cur, false);
-        KS_CUDA(cudaGetLastError());
-        return KS_OK;
-    }
     const int rc = ensure_graph(ctx, k_steps);
     if (rc) return rc;
-    KS_CUDA(cudaGraphLaunch(ctx->graph_exec[ctx->cur], ctx->stream));
+    const bool use_graph = ctx->steps_per_graph > 0 && k_steps == ctx->steps_per_graph && ctx->graph_exec[ctx->cur];
+    ctx->launched_spec = use_graph ? ctx->graph_spec[ctx->cur] : ctx->chunk_spec;
+    if (use_graph) {
+        KS_CUDA(cudaGraphLaunch(ctx->graph_exec[ctx->cur], ctx->stream));
+    } else {
+        enqueue_chunk(ctx, k_steps, ctx->cur, false);
+        KS_CUDA(cudaGetLastError());
+    }
     return KS_OK;
 }
 
@@ -737,8 +751,10 @@ int run_chunk_dev(ks_ctx* ctx, int k_steps) {
     double t_end = 0.0;
     fill_params(ctx, k_steps, ctx->t, ctx->steps_done, &t_end);
     if ((rc = plan_records(ctx, k_steps))) return rc;
-    if ((rc = ensure_graph(ctx, k_steps))) return rc;
-    if (ctx->profiling) KS_CUDA(cudaEventRecord(ctx->ev_chunk[0], ctx->stream));
+    if (ctx->profiling) {
+        if ((rc = ensure_graph(ctx, k_steps, true))) return rc;
+        KS_CUDA(cudaEventRecord(ctx->ev_chunk[0], ctx->stream));
+    }
     const HostClock::time_point hl = HostClock::now();
     ctx->timing.host_prep_ms += host_ms(h0, hl);
     rc = launch_chunk(ctx, k_steps);
@@ -762,8 +778,7 @@ int run_chunk_dev(ks_ctx* ctx, int k_steps) {
                                               "in the step, or more breakup records in one chunk than " +
                                               std::to_string(ctx->b.sbm_events_cap));
     // Conjunction records, ordered on the device; those of the void step are dropped.
-    int64_t have = (ctx->steps_per_graph > 0 && k_steps == ctx->steps_per_graph) ? ctx->graph_spec[ctx->cur]
-                                                                                : ctx->chunk_spec;
+    int64_t have = ctx->launched_spec;
     int64_t nc = std::min<int64_t>(static_cast<int64_t>(ch.conj_count), ctx->b.conj_cap);
     if (ch.flags & ks::FLAG_CONJ_LARGE) {
         ks::launch_conj_sort(ctx->b, ctx->b.chunk, &ctx->b.params[0].t0, k_steps * ctx->dt, false, ctx->stream);
@@ -867,11 +882,12 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
     double t_end = 0.0;
     fill_params(ctx, k_steps, ctx->t, ctx->steps_done, &t_end);  // uploaded by the chunk itself
     if ((rc = plan_chunk(ctx, k_steps))) return rc;
-    const bool use_graph = ctx->steps_per_graph > 0 && k_steps == ctx->steps_per_graph;
     // A new graph is built before the chunk's start is recorded, so that the
     // chunk's device time holds no wait for the host.
-    if ((rc = ensure_graph(ctx, k_steps))) return rc;
-    if (ctx->profiling) KS_CUDA(cudaEventRecord(ctx->ev_chunk[0], ctx->stream));
+    if (ctx->profiling) {
+        if ((rc = ensure_graph(ctx, k_steps, true))) return rc;
+        KS_CUDA(cudaEventRecord(ctx->ev_chunk[0], ctx->stream));
+    }
     if (ctx->screening) {
         rc = save_checkpoint(ctx, k_steps);
         if (rc) return rc;
@@ -886,7 +902,7 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
         KS_CUDA(cudaStreamSynchronize(ctx->stream));
         ctx->timing.host_launch_ms += host_ms(hl, hs);
         ctx->timing.host_sync_ms += host_ms(hs, HostClock::now());
-        have = use_graph ? ctx->graph_spec[ctx->cur] : ctx->chunk_spec;
+        have = ctx->launched_spec;
         int flags = ctx->h_chunk->flags;
         unsigned long long max_refined = 0;
         int max_bits = 0;
@@ -960,7 +976,7 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
         rc = launch_chunk(ctx, k_steps);
         if (rc) return rc;
         KS_CUDA(cudaStreamSynchronize(ctx->stream));
-        have = ctx->steps_per_graph > 0 && k_steps == ctx->steps_per_graph ? ctx->graph_spec[ctx->cur] : ctx->chunk_spec;
+        have = ctx->launched_spec;
         if (ctx->h_chunk->flags & (ks::FLAG_CONJ_OVERFLOW | ks::FLAG_TIMEOUT | ks::FLAG_KEY_RANGE))
             return fail(ctx, KS_ERR_STATE, "replay to the first collision step overflowed");
     }
@@ -1711,7 +1727,7 @@ int ks_set_tuning(ks_ctx* ctx, const char* key, int64_t value) {
         }
     } else if (k == "box_min_rows" && value >= 0 && value <= 33) ctx->tune.box_min_rows = static_cast<int>(value);
     else if (k == "prop_block" && value >= 32 && value <= 128 && value % 32 == 0) ctx->tune.prop_block = static_cast<int>(value);
-    else if (k == "item_col_blocks" && value >= 1 && value <= 64) ctx->tune.item_col_blocks = static_cast<int>(value);
+    else if (k == "item_col_blocks" && value >= 0 && value <= 64) ctx->tune.item_col_blocks = static_cast<int>(value);
     else if (k == "pair_gate_x2" && (value == 0 || value == 1)) ctx->tune.pair_gate_x2 = static_cast<int>(value);
     else if (k == "pair_stage2" && value >= 0 && value <= 2) ctx->tune.pair_stage2 = static_cast<int>(value);
     else if (k == "prop_min_blocks" && value >= 4 && value <= 6) ctx->tune.prop_min_blocks = static_cast<int>(value);
@@ -1763,7 +1779,7 @@ struct Knobs {
 Knobs current_knobs(const ks_ctx* ctx) {
     return Knobs{ctx->steps_per_graph, ctx->tune.pair_variant, ctx->tune.pair_blocks_per_sm, ctx->tune.subcell_bits,
                  ctx->tune.box_min_rows, static_cast<int>(std::lround(ctx->tune.cell_scale * 1000.0)),
-                 ctx->tune.prop_block, ctx->tune.item_col_blocks};
+                 ctx->tune.prop_block, ks::item_blocks(ctx->tune, ctx->n)};
 }
 
 void put_knobs(ks_ctx* ctx, const Knobs& k, const Ctrl& carry) {
@@ -1983,7 +1999,7 @@ int ks_prepare_run(ks_ctx* ctx) {
     const int cur = ctx->cur;
     for (int p = 0; p < 2 && !rc; ++p) {
         ctx->cur = p;
-        rc = ensure_graph(ctx, k);
+        rc = ensure_graph(ctx, k, true);
     }
     ctx->cur = cur;
     return rc;
