@@ -2,10 +2,11 @@
 // (ks_kernels.cu). Not part of the public C ABI.
 //
 // Device data layout (one context, capacity `cap` objects):
-//   state[2]     two FP64 buffers of cap states, 6 contiguous doubles each
-//                {rx, ry, rz, vx, vy, vz} (the reference's State), ping-ponged
-//                each step (start-of-step -> end-of-step)
-//   alive[2]     one byte per object per buffer
+//   state[3]     FP64 buffers of cap states, 6 contiguous doubles each
+//                {rx, ry, rz, vx, vy, vz} (the reference's State), taken in turn
+//                each step (start-of-step -> end-of-step); the third one where
+//                a step's refinement runs beside the next step
+//   alive[3]     one byte per object per buffer
 //   size_m       characteristic size L (m); collision radius = L/2
 //   keys/idx     cell keys (u64) and object indices (i32), two buffers each for the radix sort
 //   cells        begin offsets, keys, column-list lengths, 13 forward neighbours per cell
@@ -115,8 +116,8 @@ struct ChunkCtrl {
 
 struct DeviceBuffers {
     int64_t cap = 0;
-    double* state[2] = {nullptr, nullptr};
-    uint8_t* alive[2] = {nullptr, nullptr};
+    double* state[3] = {nullptr, nullptr, nullptr};   // the third: steps whose refinement runs beside the next step
+    uint8_t* alive[3] = {nullptr, nullptr, nullptr};
     double* size_m = nullptr;
     uint16_t* real_id = nullptr;           // realisation of each object (batches), else null
     double* ckpt_state = nullptr;
@@ -153,6 +154,7 @@ struct DeviceBuffers {
     float4* rec32 = nullptr;               // the same records in object order, written with the keys
     int* sorted_orig = nullptr;
     int2* survivors = nullptr;
+    int2* survivors2 = nullptr;            // of every other step, where a refinement runs beside the next step
     int64_t surv_cap = 0;
     ks_conjunction* conj = nullptr;
     int64_t conj_cap = 0;
@@ -232,7 +234,8 @@ struct StepArgs {
     const StepParams* sp;      // this step's inputs
     Ctrl* ctrl;                // this step's control block
     Ctrl* ctrl_next;           // next step's control block (speculation outputs)
-    int src;                   // state buffer holding the start of the step (0 or 1)
+    int src, dst;              // state buffers holding the start and the end of the step
+    int odd;                   // survivors go to survivors2
     unsigned int* hist;        // radix digit histogram the propagation fills with the keys it emits, or null
     float4* rec32;             // FP32 record of each object, written with its key (object order)
     int overlap;               // the step's kernels may start while their predecessors drain (launch_after)
@@ -351,8 +354,6 @@ void launch_refine(const DeviceBuffers& b, const StepArgs& a, ks_conjunction* co
 // The same with the pairs' end states (12 doubles a pair) and sizes (2) in the order of the survivors.
 void launch_refine_rows(const DeviceBuffers& b, const StepArgs& a, const double* ends, const double* sizes,
                         ks_conjunction* conj_out, int64_t conj_cap, ChunkCtrl* chunk, cudaStream_t stream);
-// Empties the counted build's tables, as the refinement does at its end (a step that is not refined).
-void launch_clear_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 
 // Device SBM (ks_sbm.cu). After a step's refinement: voids the rest of the
 // chunk if the step's buffers overflowed, then fragments the step's

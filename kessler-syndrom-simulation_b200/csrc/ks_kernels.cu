@@ -2014,7 +2014,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_pairs_split(StepArgs a, 
                                                         const float4* __restrict__ sorted32,
                                                         const int* __restrict__ orig,
                                                         const int2* __restrict__ col_tab, const int4* __restrict__ items,
-                                                        int64_t items_cap, int2* __restrict__ surv, int64_t surv_cap) {
+                                                        int64_t items_cap, int2* __restrict__ surv, int64_t surv_cap,
+                                                        unsigned long long* __restrict__ hk,
+                                                        unsigned long long* __restrict__ occ, int64_t slots) {
     after_predecessor();
     __shared__ float4 rows32[kWarps][32][2];
     // The same rows in pairs, components interleaved, for the packed gate.
@@ -2029,6 +2031,14 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_pairs_split(StepArgs a, 
     __shared__ unsigned short pq[kWarps][64];
     __shared__ int2 fq[kWarps][64];
     if (step_void(a.ctrl)) return;
+    // The counted build's hash and occupancy words, no longer read, left
+    // empty for the next step (slots 0: another build, which empties the hash
+    // itself).
+    for (int64_t q = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; q < slots / 2;
+         q += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        reinterpret_cast<ulonglong2*>(hk)[q] = make_ulonglong2(kEmpty, kEmpty);
+        if (q < slots / 8) reinterpret_cast<ulonglong2*>(occ)[q] = make_ulonglong2(0, 0);
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lanes_below = (1u << lane) - 1u;
     // Items of the list's front, then those of its back (counted cell build).
@@ -2211,19 +2221,9 @@ __global__ void __launch_bounds__(kBlock) k_refine_exact(StepArgs a, const doubl
                                                          const double* __restrict__ size_m,
                                                          const int2* __restrict__ surv, int64_t surv_cap,
                                                          ks_conjunction* __restrict__ out, int64_t cap,
-                                                         ChunkCtrl* chunk, unsigned long long* __restrict__ hk,
-                                                         unsigned long long* __restrict__ occ, int64_t slots,
-                                                         int by_pair) {
+                                                         ChunkCtrl* chunk, int by_pair) {
     after_predecessor();
     if (step_void(a.ctrl)) return;
-    // The counted build's hash and occupancy words, no longer read, left
-    // empty for the next step (slots 0: another build, which empties the hash
-    // itself).
-    for (int64_t q = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; q < slots / 2;
-         q += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        reinterpret_cast<ulonglong2*>(hk)[q] = make_ulonglong2(kEmpty, kEmpty);
-        if (q < slots / 8) reinterpret_cast<ulonglong2*>(occ)[q] = make_ulonglong2(0, 0);
-    }
     const unsigned long long ns = min(a.ctrl->refined, static_cast<unsigned long long>(surv_cap));
     const double t0 = a.sp->t0;
     const double s_hi = xsub(1.0, 1e-9);
@@ -3891,8 +3891,8 @@ void launch_seed_ctrl(const DeviceBuffers& b, int n, int src, Ctrl* target, int 
 
 void launch_propagate(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
     auto go = [&](auto kernel, int grid) {
-        launch_after(a.overlap && !a.hist, kernel, grid, a.tune.prop_block, stream, a, b.state[a.src], b.state[1 - a.src],
-                     b.alive[a.src], b.alive[1 - a.src], b.keys[0]);
+        launch_after(a.overlap && !a.hist, kernel, grid, a.tune.prop_block, stream, a, b.state[a.src], b.state[a.dst],
+                     b.alive[a.src], b.alive[a.dst], b.keys[0]);
     };
     if (a.precision == KS_PRECISION_SPLIT) {
         go(k_propagate_split, grid_for_block(a.n, 5 * kPropBlock / a.tune.prop_block, a.tune.prop_block));
@@ -3939,11 +3939,11 @@ void launch_clear_alive(uint8_t* alive, const int64_t* idx, int count, cudaStrea
 }
 
 void launch_screen_keys(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
-    k_screen_keys<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a, b.state[a.src], b.alive[1 - a.src], b.keys[0]);
+    k_screen_keys<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a, b.state[a.src], b.alive[a.dst], b.keys[0]);
 }
 
 void launch_fix_keys(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
-    k_fix_keys<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a, b.state[a.src], b.alive[1 - a.src], b.keys[0]);
+    k_fix_keys<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a, b.state[a.src], b.alive[a.dst], b.keys[0]);
 }
 
 void launch_sort(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
@@ -4159,11 +4159,14 @@ bool cells_counted(const DeviceBuffers& b, const StepArgs& a) {
 }
 
 namespace {
+int2* survivors_of(const DeviceBuffers& b, const StepArgs& a) { return a.odd ? b.survivors2 : b.survivors; }
+
 // Hash slots of a step's counted build: a power of two above 5/4 of the
-// objects (above 5/2 up to a million: the smaller tables stay in L2 at that
-// size, and a half as crowded one loses fewer exchanges), at most the whole table.
+// objects, above 5/2 for small populations, whose objects all arrive at once
+// and lose fewer exchanges in a half as crowded table (the larger table costs
+// its clearing: 41 MB a step at a million objects), at most the whole table.
 int64_t count_slots(const DeviceBuffers& b, int n) {
-    const int64_t want = n <= (1 << 20) ? 5 * static_cast<int64_t>(n) / 2 : 5 * static_cast<int64_t>(n) / 4;
+    const int64_t want = n <= (1 << 17) ? 5 * static_cast<int64_t>(n) / 2 : 5 * static_cast<int64_t>(n) / 4;
     int64_t slots = 64;
     while (slots < b.hash_cap && slots < want) slots <<= 1;
     return slots;
@@ -4192,11 +4195,11 @@ void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, 
     f.per = item_blocks(a.tune, a.n);
     const bool o = a.overlap != 0;
     launch_after(o && !screen, screen ? k_place<true> : k_place<false>, grid_for(a.n, 8), kBlock, stream, a, f,
-                 b.state[a.src], b.alive[1 - a.src]);
+                 b.state[a.src], b.alive[a.dst]);
     launch_after(o, k_number, grid_for(static_cast<int64_t>(f.slots / 4), 6), kBlock, stream, a, f);
     launch_after(o, k_scatter, grid_for(a.n, 8), kBlock, stream, a, f);
     launch_after(o, k_cells, grid_for_block(4 * static_cast<int64_t>(a.n), kCellBlocksPerSm, kCellBlock), kCellBlock, stream,
-                 a, f, b.state[a.src], b.sorted32, b.sorted_orig, b.survivors, b.surv_cap);
+                 a, f, b.state[a.src], b.sorted32, b.sorted_orig, survivors_of(b, a), b.surv_cap);
 }
 
 void launch_pairs(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
@@ -4208,8 +4211,8 @@ void launch_pairs(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream
         const int bps = a.tune.pair_blocks_per_sm > 0 ? a.tune.pair_blocks_per_sm : 4;
         launch_after(a.overlap && cells_counted(b, a),
                      bps >= 5 ? k_pairs_split<5> : bps == 4 ? k_pairs_split<4> : k_pairs_split<3>, sm_count() * bps, kBlock,
-                     stream, a, b.state[a.src], b.sorted32, b.sorted_orig, b.col_tab, b.items, b.items_cap, b.survivors,
-                     b.surv_cap);
+                     stream, a, b.state[a.src], b.sorted32, b.sorted_orig, b.col_tab, b.items, b.items_cap, survivors_of(b, a),
+                     b.surv_cap, b.hash_keys, b.occ, cells_counted(b, a) ? count_slots(b, a.n) : 0);
         return;
     }
     const int bps = a.tune.pair_blocks_per_sm > 0 ? a.tune.pair_blocks_per_sm : (a.tune.pair_variant == 1 ? 3 : 2);
@@ -4225,26 +4228,18 @@ namespace {
 void refine(const DeviceBuffers& b, const StepArgs& a, const double* after, const double* size_m, bool by_pair,
             ks_conjunction* conj_out, int64_t conj_cap, ChunkCtrl* chunk, cudaStream_t stream) {
     launch_after(a.overlap != 0, k_refine_exact, sm_count() * 2, kBlock, stream, a, b.state[a.src], after, size_m,
-                 b.survivors, b.surv_cap, conj_out, conj_cap, chunk, b.hash_keys, b.occ,
-                 cells_counted(b, a) ? count_slots(b, a.n) : 0, by_pair ? 1 : 0);
+                 survivors_of(b, a), b.surv_cap, conj_out, conj_cap, chunk, by_pair ? 1 : 0);
 }
 }  // namespace
 
 void launch_refine(const DeviceBuffers& b, const StepArgs& a, ks_conjunction* conj_out, int64_t conj_cap,
                    ChunkCtrl* chunk, cudaStream_t stream) {
-    refine(b, a, b.state[1 - a.src], b.size_m, false, conj_out, conj_cap, chunk, stream);
+    refine(b, a, b.state[a.dst], b.size_m, false, conj_out, conj_cap, chunk, stream);
 }
 
 void launch_refine_rows(const DeviceBuffers& b, const StepArgs& a, const double* ends, const double* sizes,
                         ks_conjunction* conj_out, int64_t conj_cap, ChunkCtrl* chunk, cudaStream_t stream) {
     refine(b, a, ends, sizes, true, conj_out, conj_cap, chunk, stream);
-}
-
-void launch_clear_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
-    if (!cells_counted(b, a)) return;
-    const size_t slots = static_cast<size_t>(count_slots(b, a.n));
-    cudaMemsetAsync(b.hash_keys, 0xFF, sizeof(unsigned long long) * slots, stream);
-    cudaMemsetAsync(b.occ, 0, sizeof(unsigned long long) * (slots / 4), stream);
 }
 
 cudaError_t measure_fp64(double* addmul_per_s, double* fma_per_s, cudaStream_t stream) {

@@ -201,6 +201,8 @@ int screen_noalloc(int64_t n, const double* before, const double* after, const u
 
     ks::StepArgs a{};
     a.tune.item_col_blocks = 16;  // the fixed item list is sized for items of this length
+    a.src = 0;
+    a.dst = 1;
     a.fc.neg_mu_earth = -ks::kMuEarth;
     a.fc.k_j2 = ks::j2_numerator();
     a.fc.mu_moon = ks::kMuMoon;

@@ -644,11 +644,11 @@ void launch_sbm_step(const DeviceBuffers& b, const StepArgs& a, const SbmArgs& s
     const int cap = b.coll_cap;
     const int blocks = sm_count() * 2;
     k_sbm_order<<<1, kOrderThreads, kOrderSmem, stream>>>(a, b.sbm_order, b.sbm_misc);
-    k_sbm_parents<<<blocks, 128, 0, stream>>>(a, b.state[a.src], b.state[1 - a.src], b.size_m, b.mass_kg, a.real_id,
+    k_sbm_parents<<<blocks, 128, 0, stream>>>(a, b.state[a.src], b.state[a.dst], b.size_m, b.mass_kg, a.real_id,
                                               b.sbm_order, b.sbm_work, b.sbm_first);
-    k_sbm_simple<<<blocks, 128, 0, stream>>>(a, s, b.alive[1 - a.src], b.mass_kg, b.sbm_work, b.sbm_first,
+    k_sbm_simple<<<blocks, 128, 0, stream>>>(a, s, b.alive[a.dst], b.mass_kg, b.sbm_work, b.sbm_first,
                                              b.sbm_misc, b.sbm_pending);
-    k_sbm_conflicts<<<1, kOrderThreads, kConflictSmem, stream>>>(a, s, b.alive[1 - a.src], b.mass_kg, b.sbm_work,
+    k_sbm_conflicts<<<1, kOrderThreads, kConflictSmem, stream>>>(a, s, b.alive[a.dst], b.mass_kg, b.sbm_work,
                                                                  b.sbm_misc, b.sbm_pending);
     k_sbm_number<<<1, kOrderThreads, kNumberSmem, stream>>>(a, b.sbm_work, b.sbm_next_event, b.sbm_first,
                                                            b.sbm_events_cap, s.realisations);
@@ -657,7 +657,7 @@ void launch_sbm_step(const DeviceBuffers& b, const StepArgs& a, const SbmArgs& s
     count_only.fc = a.fc;
     k_sbm_fragments<<<blocks * 2, 32 * kFragWarps, 0, stream>>>(a.ctrl, cap, s, b.sbm_work, count_only, a.chunk);
     k_sbm_place<<<1, 1024, 0, stream>>>(a.ctrl, cap, s, b.sbm_work, b.sbm_events, b.n_live, a.chunk);
-    const FragmentSink sink = make_sink(b, b.state[1 - a.src], b.alive[1 - a.src], a.ctrl_next, a.sp, a.dt, a.fc);
+    const FragmentSink sink = make_sink(b, b.state[a.dst], b.alive[a.dst], a.ctrl_next, a.sp, a.dt, a.fc);
     k_sbm_fragments<<<blocks * 2, 32 * kFragWarps, 0, stream>>>(a.ctrl, cap, s, b.sbm_work, sink, a.chunk);
 }
 

@@ -77,3 +77,16 @@ def test_counted_cells_equal_the_sorted_builds(engine, ks, precision):
         assert np.array_equal(other[0], runs[0][0]) and np.array_equal(other[1], runs[0][1])
         assert_same_conj(other[2], runs[0][2])
         assert_same_stats(other[3], runs[0][3])
+
+
+@pytest.mark.parametrize("spg,chunks", [(0, [1, 2, 3, 4, 5, 6]), (4, [4, 4, 1, 4, 4, 4]), (5, [5, 5, 5, 2, 5])])
+def test_refinement_beside_the_next_step(engine, oracle, ks, spg, chunks):
+    """Steps whose refinement runs on a second stream while the next step
+    overwrites buffers, over chunks of every parity, with records in every step."""
+    st, sz, al = ks.generate_population(505, 5000, 30000, 8, 3600.0)
+    got = run_engine(engine, st, sz, al, sum(chunks), spg=spg, chunks=chunks)
+    want = oracle.run(st, sz, al, steps=sum(chunks))
+    assert len(want[2]) > 20
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    assert_same_conj(got[2], want[2])
+    assert_same_stats(got[3], want[3])
