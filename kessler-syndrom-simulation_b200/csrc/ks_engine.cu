@@ -89,7 +89,7 @@ struct ks_ctx {
     size_t frag_scratch_bytes = 0;
     bool pack_keys = true;     // object index packed below the cell key in the sort keys
     int64_t max_step_conj = 0; // most conjunction records of one step so far (record buffer sizing)
-    bool conj_small = false;   // chunks order their records in one block (few expected)
+    bool conj_small = false;   // chunks order their records in one launch (few expected)
     int64_t chunk_spec = 0;    // records a chunk copies back with its control blocks
     int64_t graph_spec[2] = {0, 0};  // the same, as captured in graph_exec[]
     int64_t graph_n[2] = {-1, -1};   // population size graph_exec[] was captured for
@@ -789,7 +789,7 @@ int plan_records(ks_ctx* ctx, int k_steps) {
         const int64_t want = std::min<int64_t>(ctx->max_step_conj * span * 5 / 4 + 256, int64_t(1) << 30);
         if (want > ctx->b.conj_cap && (rc = ensure_conj(ctx, want))) return rc;
     }
-    // One-block ordering of the records where the chunk should hold few.
+    // One-launch ordering of the records where the chunk should hold few.
     const bool small = ctx->screening && ctx->max_step_conj > 0 &&
                        ctx->max_step_conj * k_steps * 5 / 4 + 256 <= ks::kConjSmall;
     if (small != ctx->conj_small) {
@@ -1016,7 +1016,7 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
     for (int cut = 0;; ++cut) {
         nc = static_cast<int64_t>(ctx->h_chunk->conj_count);
         if (ctx->h_chunk->flags & ks::FLAG_CONJ_LARGE) {
-            // More records than the one-block ordering takes: the multi-block sort.
+            // More records than the one-launch ordering takes: the multi-block sort.
             ks::launch_conj_sort(ctx->b, ctx->b.chunk, &ctx->b.params[0].t0, k_steps * ctx->dt, false, ctx->stream);
             KS_CUDA(cudaMemcpyAsync(ctx->h_chunk, ctx->b.chunk, sizeof(ks::ChunkCtrl), cudaMemcpyDeviceToHost,
                                     ctx->stream));

@@ -66,7 +66,7 @@ enum : int {
     FLAG_TIMEOUT = 32,       // a bounded device-side wait gave up
     FLAG_KEYS_REBUILT = 64,  // k_fix_keys rebuilt the keys: their digit histogram is recounted
     FLAG_PACK_WIDTH = 128,   // cell key + dead flag + object index do not fit 64 bits: sort unpacked
-    FLAG_CONJ_LARGE = 256,   // more records than the one-block ordering takes: ordered by the multi-block sort
+    FLAG_CONJ_LARGE = 256,   // more records than the one-launch ordering takes: ordered by the multi-block sort
     FLAG_COLL_OVERFLOW = 512,   // device SBM: more collisions in one step than its event buffer holds
     FLAG_POP_BUDGET = 1024,     // device SBM: fragments would pass the population's capacity
     FLAG_HALTED = 2048,         // device SBM: an earlier step of the chunk was left void; this step does nothing
@@ -344,7 +344,7 @@ void launch_pairs(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream
 // whose TCAs share a 32-bit key keep their append order; the host finishes
 // the (t, i, j) order). t_start: device address of the chunk's first step
 // start time; span_s: the chunk's duration.
-// Records ordered by one block in shared memory (chunks expected to hold few).
+// Records ordered in one launch, by enumeration (chunks expected to hold few).
 constexpr int kConjSmall = 16384;
 void launch_conj_sort(const DeviceBuffers& b, ChunkCtrl* chunk, const double* t_start, double span_s, bool small,
                       cudaStream_t stream);

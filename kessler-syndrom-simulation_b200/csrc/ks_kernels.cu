@@ -3997,10 +3997,6 @@ __global__ void __launch_bounds__(kBlock) k_conj_gather(const ks_conjunction* __
         out[q] = conj[static_cast<int>(order[q] & mask)];
 }
 
-// Up to kConjSmall records of a chunk ordered by one block: the keys of
-// k_conj_keys (14 index bits here) sorted by a bitonic network in shared
-// memory, then the records gathered. With more records it sets
-// FLAG_CONJ_LARGE and leaves them to the multi-block sort.
 // (t, i, j) order of records (src/core/collision.cpp:743-747).
 __device__ __forceinline__ bool conj_before(const ks_conjunction& a, const ks_conjunction& b) {
     if (a.t != b.t) return a.t < b.t;
@@ -4044,50 +4040,58 @@ __global__ void __launch_bounds__(kBlock) k_conj_ties(const unsigned long long* 
         order_tie_run(q, n, key_at, out, chunk);
 }
 
-__global__ void __launch_bounds__(1024) k_conj_sort_small(const ks_conjunction* __restrict__ conj, int64_t cap,
-                                                          ChunkCtrl* chunk, const double* __restrict__ t_start,
-                                                          double span_s, ks_conjunction* __restrict__ out) {
-    extern __shared__ unsigned long long sk[];
-    const int n = static_cast<int>(min(chunk->conj_count, static_cast<unsigned long long>(cap)));
+// Up to kConjSmall records of a chunk ordered by (t, i, j) in one launch, by
+// enumeration: a record's place is the number of records before it. P lanes
+// share a record, each counting through every P-th of all keys in shared
+// memory, with P such that the launch's threads are all in use; n^2 comparisons
+// take under 3 us for 2 500 records and some 30 us for 16 384, where one block's
+// bitonic network over the padded keys, then runs of tied keys ordered one by
+// one, took 340 us (2 500 records of a 16-step chunk of a breakup ensemble).
+// With more records it sets FLAG_CONJ_LARGE and leaves them to the multi-block
+// sort.
+__global__ void __launch_bounds__(kBlock) k_conj_rank(const ks_conjunction* __restrict__ conj, int64_t cap,
+                                                      ChunkCtrl* chunk, ks_conjunction* __restrict__ out) {
+    constexpr int kTile = 1024;
+    __shared__ unsigned long long sh_t[kTile], sh_ij[kTile];
+    const int n = static_cast<int>(min(chunk->conj_count, static_cast<unsigned long long>(min(cap, static_cast<int64_t>(kConjSmall + 1)))));
     if (n > kConjSmall) {
-        if (threadIdx.x == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
             chunk->sort_n = 0;
             atomicOr(&chunk->flags, FLAG_CONJ_LARGE);
         }
         return;
     }
-    if (threadIdx.x == 0) chunk->sort_n = n;
-    int m = 2;
-    while (m < n) m <<= 1;
-    const double t0 = *t_start;
-    for (int q = threadIdx.x; q < m; q += blockDim.x) {
-        unsigned long long key = ~0ull;  // padding sorts last
-        if (q < n) {
-            const double f = xmul(xdiv(xsub(conj[q].t, t0), span_s), 4294967296.0);
-            const double c = fmin(fmax(floor(f), 0.0), 4294967295.0);
-            key = (static_cast<unsigned long long>(c) << 14) | static_cast<unsigned long long>(q);
+    if (blockIdx.x == 0 && threadIdx.x == 0) chunk->sort_n = n;
+    int P = 1;
+    while (P < 32 && 2 * P * n <= static_cast<int>(gridDim.x) * kBlock) P *= 2;
+    const int per_block = kBlock / P, part = threadIdx.x & (P - 1);
+    for (int q0 = blockIdx.x * per_block; q0 < n; q0 += gridDim.x * per_block) {
+        const int q = q0 + static_cast<int>(threadIdx.x) / P;
+        const bool have = q < n;
+        unsigned long long t = 0, ij = 0;
+        if (have) {
+            t = enc_double(conj[q].t);
+            ij = (static_cast<unsigned long long>(static_cast<unsigned int>(conj[q].i)) << 32) | static_cast<unsigned int>(conj[q].j);
         }
-        sk[q] = key;
-    }
-    __syncthreads();
-    for (int k = 2; k <= m; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < m; i += blockDim.x) {
-                const int p = i ^ j;
-                if (p > i) {
-                    const unsigned long long a = sk[i], b = sk[p];
-                    if ((a > b) == ((i & k) == 0)) {
-                        sk[i] = b;
-                        sk[p] = a;
-                    }
-                }
+        int rank = 0;
+        for (int r0 = 0; r0 < n; r0 += kTile) {
+            __syncthreads();
+            const int m = min(kTile, n - r0);
+            for (int r = threadIdx.x; r < m; r += kBlock) {
+                const ks_conjunction& c = conj[r0 + r];
+                sh_t[r] = enc_double(c.t);
+                sh_ij[r] = (static_cast<unsigned long long>(static_cast<unsigned int>(c.i)) << 32) | static_cast<unsigned int>(c.j);
             }
             __syncthreads();
+            for (int r = part; r < m; r += P) {
+                const unsigned long long u = sh_t[r];
+                // Equal records, which do not occur, would keep their order.
+                if (u < t || (u == t && (sh_ij[r] < ij || (sh_ij[r] == ij && r0 + r < q)))) ++rank;
+            }
         }
-    for (int q = threadIdx.x; q < n; q += blockDim.x) out[q] = conj[static_cast<int>(sk[q] & 0x3FFFull)];
-    __syncthreads();
-    auto key_at = [&](int p) { return sk[p] >> 14; };
-    for (int q = threadIdx.x; q < n; q += blockDim.x) order_tie_run(q, n, key_at, out, chunk);
+        for (int o = P / 2; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+        if (have && part == 0) out[rank] = conj[q];
+    }
 }
 
 void launch_conj_sort(const DeviceBuffers& b, ChunkCtrl* chunk, const double* t_start, double span_s, bool small,
@@ -4095,9 +4099,7 @@ void launch_conj_sort(const DeviceBuffers& b, ChunkCtrl* chunk, const double* t_
     const int cap = static_cast<int>(b.conj_cap);
     if (cap <= 0) return;
     if (small) {
-        constexpr int kBytes = kConjSmall * sizeof(unsigned long long);
-        cudaFuncSetAttribute(k_conj_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
-        k_conj_sort_small<<<1, 1024, kBytes, stream>>>(b.conj, b.conj_cap, chunk, t_start, span_s, b.conj_sorted);
+        k_conj_rank<<<sm_count(), kBlock, 0, stream>>>(b.conj, b.conj_cap, chunk, b.conj_sorted);
         return;
     }
     constexpr int kPasses = 4;
