@@ -3465,10 +3465,10 @@ __global__ void __launch_bounds__(kCellBlock, kCellBlocksPerSm) k_cells(StepArgs
     const int n = live_n(a);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nc = min(n, static_cast<int>(static_cast<unsigned int>(ctrl->placed)));
-    // Cells per warp: 32 lanes' worth, fewer where that would leave most of
-    // the chip's warps idle and the launch as long as one warp's chain.
-    int per_warp = 32;
-    while (per_warp > 8 && nc < per_warp * kCellWarps * static_cast<int>(gridDim.x)) per_warp >>= 1;
+    // Cells per warp: 32 lanes' worth; fewer where that would leave warps of
+    // the grid idle, so that every warp takes one round of about as many.
+    const int warps = kCellWarps * static_cast<int>(gridDim.x);
+    const int per_warp = max(8, min(32, (nc + warps - 1) / warps));
     if (per_warp * static_cast<int>(blockIdx.x * kCellWarps) >= nc) return;
     const PairGate pg = pair_gate(a);
     const int per = f.per;
@@ -3972,8 +3972,13 @@ void launch_sort(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream)
     }
 }
 
-// Key of each of the chunk's records: floor(2^32 (t - t_start) / span),
-// clamped, a non-decreasing function of t, above the record's index.
+// floor(2^32 (t - t_start) / span), clamped: a non-decreasing function of t.
+__device__ __forceinline__ unsigned int conj_key32(double t, double t0, double span_s) {
+    const double f = xmul(xdiv(xsub(t, t0), span_s), 4294967296.0);
+    return static_cast<unsigned int>(fmin(fmax(floor(f), 0.0), 4294967295.0));
+}
+
+// Key of each of the chunk's records: conj_key32 above the record's index.
 __global__ void __launch_bounds__(kBlock) k_conj_keys(const ks_conjunction* __restrict__ conj, int64_t cap,
                                                       ChunkCtrl* chunk, const double* __restrict__ t_start,
                                                       double span_s, unsigned long long* __restrict__ keys,
@@ -3982,9 +3987,8 @@ __global__ void __launch_bounds__(kBlock) k_conj_keys(const ks_conjunction* __re
     if (blockIdx.x == 0 && threadIdx.x == 0) chunk->sort_n = n;
     const double t0 = *t_start;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        const double f = xmul(xdiv(xsub(conj[q].t, t0), span_s), 4294967296.0);
-        const double c = fmin(fmax(floor(f), 0.0), 4294967295.0);
-        keys[q] = (static_cast<unsigned long long>(c) << pack_bits) | static_cast<unsigned long long>(q);
+        keys[q] = (static_cast<unsigned long long>(conj_key32(conj[q].t, t0, span_s)) << pack_bits) |
+                  static_cast<unsigned long long>(q);
     }
 }
 
@@ -4042,17 +4046,19 @@ __global__ void __launch_bounds__(kBlock) k_conj_ties(const unsigned long long* 
 
 // Up to kConjSmall records of a chunk ordered by (t, i, j) in one launch, by
 // enumeration: a record's place is the number of records before it. P lanes
-// share a record, each counting through every P-th of all keys in shared
-// memory, with P such that the launch's threads are all in use; n^2 comparisons
-// take under 3 us for 2 500 records and some 30 us for 16 384, where one block's
-// bitonic network over the padded keys, then runs of tied keys ordered one by
-// one, took 340 us (2 500 records of a 16-step chunk of a breakup ensemble).
-// With more records it sets FLAG_CONJ_LARGE and leaves them to the multi-block
-// sort.
+// share a record, each counting through every P-th group of four of all 32-bit
+// keys (those of k_conj_keys) in shared memory, with P such that the launch's
+// threads are all in use; a record that shares its key looks at the records
+// themselves. One block's bitonic network over the padded keys, then runs of
+// tied keys ordered one by one, took 340 us for the 2 500 records of a 16-step
+// chunk of a breakup ensemble, this 5. With more records it sets
+// FLAG_CONJ_LARGE and leaves them to the multi-block sort.
 __global__ void __launch_bounds__(kBlock) k_conj_rank(const ks_conjunction* __restrict__ conj, int64_t cap,
-                                                      ChunkCtrl* chunk, ks_conjunction* __restrict__ out) {
-    constexpr int kTile = 1024;
-    __shared__ unsigned long long sh_t[kTile], sh_ij[kTile];
+                                                      ChunkCtrl* chunk, const double* __restrict__ t_start,
+                                                      double span_s, ks_conjunction* __restrict__ out) {
+    constexpr int kTile = 4096;
+    __shared__ uint4 sh[kTile / 4];
+    unsigned int* keys = reinterpret_cast<unsigned int*>(sh);
     const int n = static_cast<int>(min(chunk->conj_count, static_cast<unsigned long long>(min(cap, static_cast<int64_t>(kConjSmall + 1)))));
     if (n > kConjSmall) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -4062,31 +4068,35 @@ __global__ void __launch_bounds__(kBlock) k_conj_rank(const ks_conjunction* __re
         return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) chunk->sort_n = n;
+    const double t0 = *t_start;
     int P = 1;
     while (P < 32 && 2 * P * n <= static_cast<int>(gridDim.x) * kBlock) P *= 2;
     const int per_block = kBlock / P, part = threadIdx.x & (P - 1);
     for (int q0 = blockIdx.x * per_block; q0 < n; q0 += gridDim.x * per_block) {
         const int q = q0 + static_cast<int>(threadIdx.x) / P;
         const bool have = q < n;
-        unsigned long long t = 0, ij = 0;
-        if (have) {
-            t = enc_double(conj[q].t);
-            ij = (static_cast<unsigned long long>(static_cast<unsigned int>(conj[q].i)) << 32) | static_cast<unsigned int>(conj[q].j);
-        }
-        int rank = 0;
+        const unsigned int mine = have ? conj_key32(conj[q].t, t0, span_s) : 0u;
+        int rank = 0, same = 0;
         for (int r0 = 0; r0 < n; r0 += kTile) {
             __syncthreads();
-            const int m = min(kTile, n - r0);
-            for (int r = threadIdx.x; r < m; r += kBlock) {
-                const ks_conjunction& c = conj[r0 + r];
-                sh_t[r] = enc_double(c.t);
-                sh_ij[r] = (static_cast<unsigned long long>(static_cast<unsigned int>(c.i)) << 32) | static_cast<unsigned int>(c.j);
-            }
+            const int m = min(kTile, n - r0), groups = (m + 3) / 4;
+            for (int r = threadIdx.x; r < 4 * groups; r += kBlock)
+                keys[r] = r < m ? conj_key32(conj[r0 + r].t, t0, span_s) : 0xFFFFFFFFu;
             __syncthreads();
-            for (int r = part; r < m; r += P) {
-                const unsigned long long u = sh_t[r];
+#pragma unroll 4
+            for (int r = part; r < groups; r += P) {
+                const uint4 u = sh[r];
+                rank += (u.x < mine) + (u.y < mine) + (u.z < mine) + (u.w < mine);
+                same += (u.x == mine) + (u.y == mine) + (u.z == mine) + (u.w == mine);
+            }
+        }
+        for (int o = P / 2; o > 0; o >>= 1) same += __shfl_xor_sync(0xffffffffu, same, o);
+        if (have && same > 1) {
+            const ks_conjunction me = conj[q];
+            for (int r = part; r < n; r += P) {
+                const ks_conjunction& c = conj[r];
                 // Equal records, which do not occur, would keep their order.
-                if (u < t || (u == t && (sh_ij[r] < ij || (sh_ij[r] == ij && r0 + r < q)))) ++rank;
+                if (r != q && conj_key32(c.t, t0, span_s) == mine && (conj_before(c, me) || (r < q && !conj_before(me, c)))) ++rank;
             }
         }
         for (int o = P / 2; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
@@ -4099,7 +4109,7 @@ void launch_conj_sort(const DeviceBuffers& b, ChunkCtrl* chunk, const double* t_
     const int cap = static_cast<int>(b.conj_cap);
     if (cap <= 0) return;
     if (small) {
-        k_conj_rank<<<sm_count(), kBlock, 0, stream>>>(b.conj, b.conj_cap, chunk, b.conj_sorted);
+        k_conj_rank<<<2 * sm_count(), kBlock, 0, stream>>>(b.conj, b.conj_cap, chunk, t_start, span_s, b.conj_sorted);
         return;
     }
     constexpr int kPasses = 4;
