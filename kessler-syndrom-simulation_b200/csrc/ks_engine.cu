@@ -60,9 +60,9 @@ struct ks_ctx {
     int profiling = 0;
     int cur = 0;
     int prev = 1;   // state buffer the last step started from
-    // Refinements beside the next step: their stream, and events of pairs ready and refinements done (by step, in turn).
+    // Pairs and refinements beside the next step: their stream, and events of cells ready and refinements done (by step, in turn).
     cudaStream_t side = nullptr;
-    cudaEvent_t ev_pairs[4] = {nullptr, nullptr, nullptr, nullptr}, ev_refined[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t ev_cells[4] = {nullptr, nullptr, nullptr, nullptr}, ev_refined[4] = {nullptr, nullptr, nullptr, nullptr};
     int sort_passes = 8;
     bool has_pop = false;
     int max_chunk = 0;
@@ -179,6 +179,7 @@ void free_objects(ks_ctx* ctx) {
     dfree(b.sort_hist); dfree(b.sort_status); dfree(b.sort_ctr);
     dfree(b.cell_begin); dfree(b.cell_key); dfree(b.nbr); dfree(b.cell_len); dfree(b.col_tab); dfree(b.item_part); dfree(b.hash_keys); dfree(b.hash_vals);
     dfree(b.occ);
+    dfree(b.second.sorted32); dfree(b.second.sorted_orig); dfree(b.second.col_tab); dfree(b.second.hash_keys); dfree(b.second.occ);
     dfree(b.sorted); dfree(b.sorted32); dfree(b.rec32); dfree(b.sorted_orig); dfree(b.fused);
     b.fused_grid = 0;
     dfree(b.n_live); dfree(b.mass_kg); dfree(b.a2m); dfree(b.event_of); dfree(b.coll); dfree(b.sbm_work);
@@ -237,6 +238,15 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     KS_CUDA(cudaMalloc(&b.sorted32, sizeof(float4) * 2 * cap));
     KS_CUDA(cudaMalloc(&b.rec32, sizeof(float4) * 2 * cap));
     KS_CUDA(cudaMalloc(&b.sorted_orig, sizeof(int) * cap));
+    if (!ctx->dev_sbm) {
+        KS_CUDA(cudaMalloc(&b.second.sorted32, sizeof(float4) * 2 * cap));
+        KS_CUDA(cudaMalloc(&b.second.sorted_orig, sizeof(int) * cap));
+        KS_CUDA(cudaMalloc(&b.second.col_tab, sizeof(int2) * 16 * cap));
+        KS_CUDA(cudaMalloc(&b.second.hash_keys, sizeof(unsigned long long) * h));
+        KS_CUDA(cudaMalloc(&b.second.occ, sizeof(unsigned long long) * (h / 4)));
+        KS_CUDA(cudaMemset(b.second.hash_keys, 0xFF, sizeof(unsigned long long) * h));
+        KS_CUDA(cudaMemset(b.second.occ, 0, sizeof(unsigned long long) * (h / 4)));
+    }
     // Scratch of the fused sort + cell build, sized for this device's grid
     // (looked up here, outside any stream capture).
     if (const int fg = ks::fused_grid()) {
@@ -271,10 +281,10 @@ int ensure_survivors(ks_ctx* ctx, int64_t want) {
     if (want <= ctx->b.surv_cap) return KS_OK;
     drop_graphs(ctx);
     dfree(ctx->b.survivors);
-    dfree(ctx->b.survivors2);
+    dfree(ctx->b.second.survivors);
     ctx->b.surv_cap = 0;
     KS_CUDA(cudaMalloc(&ctx->b.survivors, sizeof(int2) * want));
-    KS_CUDA(cudaMalloc(&ctx->b.survivors2, sizeof(int2) * want));
+    KS_CUDA(cudaMalloc(&ctx->b.second.survivors, sizeof(int2) * want));
     ctx->b.surv_cap = want;
     return KS_OK;
 }
@@ -283,8 +293,10 @@ int ensure_items(ks_ctx* ctx, int64_t want) {
     if (want <= ctx->b.items_cap) return KS_OK;
     drop_graphs(ctx);
     dfree(ctx->b.items);
+    dfree(ctx->b.second.items);
     ctx->b.items_cap = 0;
     KS_CUDA(cudaMalloc(&ctx->b.items, sizeof(int4) * want));
+    KS_CUDA(cudaMalloc(&ctx->b.second.items, sizeof(int4) * want));
     ctx->b.items_cap = want;
     return KS_OK;
 }
@@ -519,15 +531,18 @@ void record_chunk_end(ks_ctx* ctx, bool capturing) {
     else cudaEventRecord(ctx->ev_chunk[1], ctx->stream);
 }
 
-// Whether the steps' refinements run on a second stream beside the next
-// steps: a refinement is a long dependent chain on few threads, or at large
-// populations FP64 work next to latency-bound kernels; nothing of the next
-// step reads its results. It needs the step's two state buffers and its list
-// of pairs to stay as they are meanwhile: a third state buffer and a second
-// list. Not with fragmentation on the device, which follows the refinement
-// inside the step, nor with per-phase timing. Catalogue hour 46.7 -> 42.4 us a
-// step, at dt 60 s 57.7 -> 51.3, 250 000 objects 192 -> 176, a million (split)
-// 465 -> 450.
+// Whether the steps' pairs and refinements run on a second stream beside the
+// next steps: nothing of the next step reads their results. A refinement is a
+// long dependent chain on few threads, the tile kernel of a small population
+// leaves most of the chip idle and that of a large one is bound by issue,
+// where the cell build is bound by latency. They need the step's two state
+// buffers, its cells and its list of pairs to stay as they are meanwhile: a
+// third state buffer and a second set of the rest. Not with fragmentation on
+// the device, which follows the refinement inside the step, nor with per-phase
+// timing. In us a step, in one stream / refinement aside / pairs too:
+// catalogue hour 46.7 / 42.4 / 38.8, at dt 60 s 57.7 / 51.3 / 44.9, 250 000
+// objects 192 / 176 / 160, a million (split) 465 / 450 / 408. (A higher priority for
+// either stream: 250 000 objects 168 -> 186 or 175.)
 bool refine_aside(ks_ctx* ctx) {
     if (!ctx->screening || ctx->dev_sbm || ctx->profiling || ctx->l2_flush_bytes > 0 || !ctx->b.state[2]) return false;
     return ks::cells_counted(ctx->b, step_args(ctx, 0, 1, 0));
@@ -573,7 +588,7 @@ void enqueue_chunk(ks_ctx* ctx, int k_steps, int src0, bool capturing) {
         if (a.hist) cudaMemsetAsync(a.hist, 0, sizeof(unsigned int) * 2 * 8 * 256, s);
         StepArgs p = a;
         if (aside) {
-            // The step writes buffer dst and the survivors of two steps ago.
+            // The step writes buffer dst and the cell set of two steps ago.
             a.odd = p.odd = k & 1;
             const int before = std::max(reader[a.dst], k - 2);
             if (before > waited) {
@@ -601,17 +616,18 @@ void enqueue_chunk(ks_ctx* ctx, int k_steps, int src0, bool capturing) {
                 ks::launch_cells(ctx->b, a, s);
                 record(ctx, k, 3, capturing);
             }
-            ks::launch_pairs(ctx->b, a, s);
-            record(ctx, k, 4, capturing);
             if (aside) {
-                cudaEventRecord(ctx->ev_pairs[k & 3], s);
-                cudaStreamWaitEvent(ctx->side, ctx->ev_pairs[k & 3], 0);
+                cudaEventRecord(ctx->ev_cells[k & 3], s);
+                cudaStreamWaitEvent(ctx->side, ctx->ev_cells[k & 3], 0);
                 StepArgs r = a;
                 r.overlap = 0;
-                ks::launch_refine(ctx->b, r, ctx->b.conj, ctx->b.conj_cap, ctx->b.chunk, ctx->side);
+                ks::launch_pairs(ctx->b, r, ctx->side);
+                ks::launch_refine(ctx->b, a, ctx->b.conj, ctx->b.conj_cap, ctx->b.chunk, ctx->side);
                 cudaEventRecord(ctx->ev_refined[k & 3], ctx->side);
                 reader[a.src] = reader[a.dst] = k;
             } else {
+                ks::launch_pairs(ctx->b, a, s);
+                record(ctx, k, 4, capturing);
                 ks::launch_refine(ctx->b, a, ctx->b.conj, ctx->b.conj_cap, ctx->b.chunk, s);
             }
             if (ctx->dev_sbm) {
@@ -1595,7 +1611,7 @@ int ks_create(int device, ks_ctx** out) {
         rc = KS_ERR_CUDA;
     if (!rc && cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess) rc = KS_ERR_CUDA;
     for (int k = 0; k < 4 && !rc; ++k)
-        if (cudaEventCreateWithFlags(&ctx->ev_pairs[k], cudaEventDisableTiming) != cudaSuccess ||
+        if (cudaEventCreateWithFlags(&ctx->ev_cells[k], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ctx->ev_refined[k], cudaEventDisableTiming) != cudaSuccess)
             rc = KS_ERR_CUDA;
     if (!rc) rc = ensure_chunk(ctx, 64);
@@ -1621,8 +1637,9 @@ void ks_destroy(ks_ctx* ctx) {
     free_objects(ctx);
     if (ctx->l2_flush) cudaFree(ctx->l2_flush);
     dfree(ctx->b.survivors);
-    dfree(ctx->b.survivors2);
+    dfree(ctx->b.second.survivors);
     dfree(ctx->b.items);
+    dfree(ctx->b.second.items);
     if (ctx->frag_scratch) cudaFree(ctx->frag_scratch);
     free_conj(ctx);
     free_plain(ctx);
@@ -1636,7 +1653,7 @@ void ks_destroy(ks_ctx* ctx) {
     for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->ev_chunk) if (e) cudaEventDestroy(e);
     for (int k = 0; k < 4; ++k) {
-        if (ctx->ev_pairs[k]) cudaEventDestroy(ctx->ev_pairs[k]);
+        if (ctx->ev_cells[k]) cudaEventDestroy(ctx->ev_cells[k]);
         if (ctx->ev_refined[k]) cudaEventDestroy(ctx->ev_refined[k]);
     }
     if (ctx->side) cudaStreamDestroy(ctx->side);

@@ -114,9 +114,20 @@ struct ChunkCtrl {
     int sort_n;                        // records ordered by the chunk's conjunction sort
 };
 
+// What a step's counted cell build leaves for its tile kernel.
+struct CellSet {
+    float4* sorted32 = nullptr;
+    int* sorted_orig = nullptr;
+    int2* col_tab = nullptr;
+    int4* items = nullptr;
+    unsigned long long* hash_keys = nullptr;
+    unsigned long long* occ = nullptr;
+    int2* survivors = nullptr;
+};
+
 struct DeviceBuffers {
     int64_t cap = 0;
-    double* state[3] = {nullptr, nullptr, nullptr};   // the third: steps whose refinement runs beside the next step
+    double* state[3] = {nullptr, nullptr, nullptr};   // the third: steps whose pairs run beside the next step
     uint8_t* alive[3] = {nullptr, nullptr, nullptr};
     double* size_m = nullptr;
     uint16_t* real_id = nullptr;           // realisation of each object (batches), else null
@@ -154,7 +165,7 @@ struct DeviceBuffers {
     float4* rec32 = nullptr;               // the same records in object order, written with the keys
     int* sorted_orig = nullptr;
     int2* survivors = nullptr;
-    int2* survivors2 = nullptr;            // of every other step, where a refinement runs beside the next step
+    CellSet second;                        // of every other step, where pairs and refinement run beside the next step
     int64_t surv_cap = 0;
     ks_conjunction* conj = nullptr;
     int64_t conj_cap = 0;
@@ -235,7 +246,7 @@ struct StepArgs {
     Ctrl* ctrl;                // this step's control block
     Ctrl* ctrl_next;           // next step's control block (speculation outputs)
     int src, dst;              // state buffers holding the start and the end of the step
-    int odd;                   // survivors go to survivors2
+    int odd;                   // cells and pairs go to the second set
     unsigned int* hist;        // radix digit histogram the propagation fills with the keys it emits, or null
     float4* rec32;             // FP32 record of each object, written with its key (object order)
     int overlap;               // the step's kernels may start while their predecessors drain (launch_after)

@@ -4171,7 +4171,10 @@ bool cells_counted(const DeviceBuffers& b, const StepArgs& a) {
 }
 
 namespace {
-int2* survivors_of(const DeviceBuffers& b, const StepArgs& a) { return a.odd ? b.survivors2 : b.survivors; }
+CellSet set_of(const DeviceBuffers& b, const StepArgs& a) {
+    if (a.odd) return b.second;
+    return CellSet{b.sorted32, b.sorted_orig, b.col_tab, b.items, b.hash_keys, b.occ, b.survivors};
+}
 
 // Hash slots of a step's counted build: a power of two above 5/4 of the
 // objects, above 5/2 for small populations, whose objects all arrive at once
@@ -4186,11 +4189,12 @@ int64_t count_slots(const DeviceBuffers& b, int n) {
 }  // namespace
 
 void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, cudaStream_t stream) {
+    const CellSet set = set_of(b, a);
     CountArgs f{};
     f.keys = b.keys[0];
-    f.hk = b.hash_keys;
+    f.hk = set.hash_keys;
     f.slots = static_cast<unsigned long long>(count_slots(b, a.n));
-    f.occ = b.occ;
+    f.occ = set.occ;
     f.shift = 64;
     for (unsigned long long q = f.slots / 4; q > 1; q >>= 1) --f.shift;
     f.cbits = a.pack_bits + 1;  // a count of all n objects needs one bit more than an index
@@ -4198,11 +4202,11 @@ void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, 
     f.span = reinterpret_cast<int2*>(b.sorted);
     f.cell_key = b.cell_key;
     f.cell_span = reinterpret_cast<int2*>(b.nbr);
-    f.sorted_orig = b.sorted_orig;
-    f.sorted32 = b.sorted32;
+    f.sorted_orig = set.sorted_orig;
+    f.sorted32 = set.sorted32;
     f.rec32 = b.rec32;
-    f.col_tab = b.col_tab;
-    f.items = b.items;
+    f.col_tab = set.col_tab;
+    f.items = set.items;
     f.items_cap = b.items_cap;
     f.per = item_blocks(a.tune, a.n);
     const bool o = a.overlap != 0;
@@ -4211,20 +4215,21 @@ void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, 
     launch_after(o, k_number, grid_for(static_cast<int64_t>(f.slots / 4), 6), kBlock, stream, a, f);
     launch_after(o, k_scatter, grid_for(a.n, 8), kBlock, stream, a, f);
     launch_after(o, k_cells, grid_for_block(4 * static_cast<int64_t>(a.n), kCellBlocksPerSm, kCellBlock), kCellBlock, stream,
-                 a, f, b.state[a.src], b.sorted32, b.sorted_orig, survivors_of(b, a), b.surv_cap);
+                 a, f, b.state[a.src], set.sorted32, set.sorted_orig, set.survivors, b.surv_cap);
 }
 
 void launch_pairs(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
     // Default: the resident block count of each kernel.
     if (f32_records(a)) {
+        const CellSet set = set_of(b, a);
         // Register budget for 3 resident blocks per SM (80 registers), for 4
         // (64; the default: the higher occupancy outweighs a few spilled
         // registers) or for 5 (48; the most its shared memory allows).
         const int bps = a.tune.pair_blocks_per_sm > 0 ? a.tune.pair_blocks_per_sm : 4;
         launch_after(a.overlap && cells_counted(b, a),
                      bps >= 5 ? k_pairs_split<5> : bps == 4 ? k_pairs_split<4> : k_pairs_split<3>, sm_count() * bps, kBlock,
-                     stream, a, b.state[a.src], b.sorted32, b.sorted_orig, b.col_tab, b.items, b.items_cap, survivors_of(b, a),
-                     b.surv_cap, b.hash_keys, b.occ, cells_counted(b, a) ? count_slots(b, a.n) : 0);
+                     stream, a, b.state[a.src], set.sorted32, set.sorted_orig, set.col_tab, set.items, b.items_cap, set.survivors,
+                     b.surv_cap, set.hash_keys, set.occ, cells_counted(b, a) ? count_slots(b, a.n) : 0);
         return;
     }
     const int bps = a.tune.pair_blocks_per_sm > 0 ? a.tune.pair_blocks_per_sm : (a.tune.pair_variant == 1 ? 3 : 2);
@@ -4240,7 +4245,7 @@ namespace {
 void refine(const DeviceBuffers& b, const StepArgs& a, const double* after, const double* size_m, bool by_pair,
             ks_conjunction* conj_out, int64_t conj_cap, ChunkCtrl* chunk, cudaStream_t stream) {
     launch_after(a.overlap != 0, k_refine_exact, sm_count() * 2, kBlock, stream, a, b.state[a.src], after, size_m,
-                 survivors_of(b, a), b.surv_cap, conj_out, conj_cap, chunk, by_pair ? 1 : 0);
+                 set_of(b, a).survivors, b.surv_cap, conj_out, conj_cap, chunk, by_pair ? 1 : 0);
 }
 }  // namespace
 
