@@ -61,8 +61,9 @@ struct ks_ctx {
     int cur = 0;
     int prev = 1;   // state buffer the last step started from
     // Pairs and refinements beside the next step: their stream, and events of cells ready and refinements done (by step, in turn).
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev_cells[4] = {nullptr, nullptr, nullptr, nullptr}, ev_refined[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaStream_t ahead = nullptr, side = nullptr;
+    cudaEvent_t ev_start = nullptr, ev_prop[4] = {nullptr, nullptr, nullptr, nullptr},
+                ev_cells[4] = {nullptr, nullptr, nullptr, nullptr}, ev_refined[4] = {nullptr, nullptr, nullptr, nullptr};
     int sort_passes = 8;
     bool has_pop = false;
     int max_chunk = 0;
@@ -180,6 +181,7 @@ void free_objects(ks_ctx* ctx) {
     dfree(b.cell_begin); dfree(b.cell_key); dfree(b.nbr); dfree(b.cell_len); dfree(b.col_tab); dfree(b.item_part); dfree(b.hash_keys); dfree(b.hash_vals);
     dfree(b.occ);
     dfree(b.second.sorted32); dfree(b.second.sorted_orig); dfree(b.second.col_tab); dfree(b.second.hash_keys); dfree(b.second.occ);
+    dfree(b.second.keys); dfree(b.second.rec32);
     dfree(b.sorted); dfree(b.sorted32); dfree(b.rec32); dfree(b.sorted_orig); dfree(b.fused);
     b.fused_grid = 0;
     dfree(b.n_live); dfree(b.mass_kg); dfree(b.a2m); dfree(b.event_of); dfree(b.coll); dfree(b.sbm_work);
@@ -241,6 +243,8 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     if (!ctx->dev_sbm) {
         KS_CUDA(cudaMalloc(&b.second.sorted32, sizeof(float4) * 2 * cap));
         KS_CUDA(cudaMalloc(&b.second.sorted_orig, sizeof(int) * cap));
+        KS_CUDA(cudaMalloc(&b.second.keys, sizeof(unsigned long long) * cap));
+        KS_CUDA(cudaMalloc(&b.second.rec32, sizeof(float4) * 2 * cap));
         KS_CUDA(cudaMalloc(&b.second.col_tab, sizeof(int2) * 16 * cap));
         KS_CUDA(cudaMalloc(&b.second.hash_keys, sizeof(unsigned long long) * h));
         KS_CUDA(cudaMalloc(&b.second.occ, sizeof(unsigned long long) * (h / 4)));
@@ -568,6 +572,59 @@ std::vector<int> state_turns(ks_ctx* ctx, int k_steps, int src0) {
     return buf;
 }
 
+// The steps of a chunk, a stream each for propagation, cell build (the
+// context's stream) and pairs with refinement. A step's propagation waits for
+// the last reader of the state buffer it writes and for the cell build that
+// read the keys and records it replaces, its cell build for the propagation
+// and for the pairs that used its set two steps ago, its pairs for the cells.
+// The propagation shares the cell build's stream at sizes where its blocks,
+// which fill the chip for longer than a cell kernel takes, only displace that
+// build (250 000 objects 165 us a step, on a stream of its own 178; catalogue
+// hour 38.9 and 35.1, dt 60 s 45.2 and 41.1, a million FP64 427 and 406, split
+// 381 and 366, the ensemble 732 and 706).
+void enqueue_aside(ks_ctx* ctx, int k_steps, int src0) {
+    const bool own = ctx->n < (1 << 17) || ctx->n >= (1 << 19);
+    cudaStream_t s = ctx->stream, p = own ? ctx->ahead : s, d = ctx->side;
+    const std::vector<int> buf = state_turns(ctx, k_steps, src0);
+    int reader[3] = {-1, -1, -1};        // the last step whose kernels read the buffer
+    int waited_p = -1, waited_s = -1;    // refinements up to this step's are done for the stream
+    if (own) {
+        cudaEventRecord(ctx->ev_start, s);
+        cudaStreamWaitEvent(p, ctx->ev_start, 0);
+    }
+    for (int k = 0; k < k_steps; ++k) {
+        StepArgs a = step_args(ctx, k, k_steps, buf[k], buf[k + 1]);
+        a.aside = own;
+        a.odd = k & 1;
+        if (a.odd) a.rec32 = ctx->b.second.rec32;
+        StepArgs alone = a;   // for kernels that follow an event of another stream
+        alone.overlap = 0;
+        const int before = own ? reader[a.dst] : std::max(reader[a.dst], k - 2);
+        if (before > waited_p) {
+            waited_p = before;
+            cudaStreamWaitEvent(p, ctx->ev_refined[waited_p & 3], 0);
+        }
+        if (own && k > 1) cudaStreamWaitEvent(p, ctx->ev_cells[(k - 2) & 3], 0);
+        ks::launch_propagate(ctx->b, alone, p);
+        if (own) {
+            cudaEventRecord(ctx->ev_prop[k & 3], p);
+            cudaStreamWaitEvent(s, ctx->ev_prop[k & 3], 0);
+            if (k - 2 > waited_s) {
+                waited_s = k - 2;
+                cudaStreamWaitEvent(s, ctx->ev_refined[waited_s & 3], 0);
+            }
+        }
+        ks::launch_count_cells(ctx->b, a, false, s);
+        cudaEventRecord(ctx->ev_cells[k & 3], s);
+        cudaStreamWaitEvent(d, ctx->ev_cells[k & 3], 0);
+        ks::launch_pairs(ctx->b, alone, d);
+        ks::launch_refine(ctx->b, a, ctx->b.conj, ctx->b.conj_cap, ctx->b.chunk, d);
+        cudaEventRecord(ctx->ev_refined[k & 3], d);
+        reader[a.src] = reader[a.dst] = k;
+    }
+    cudaStreamWaitEvent(s, ctx->ev_refined[(k_steps - 1) & 3], 0);
+}
+
 // A chunk in stream order: its step parameters up (from h_params), set-up
 // (with the checkpoint of the carried speculation), the steps, the ordering
 // of its records, and its control blocks and first chunk_spec records back to
@@ -576,68 +633,47 @@ void enqueue_chunk(ks_ctx* ctx, int k_steps, int src0, bool capturing) {
     cudaStream_t s = ctx->stream;
     cudaMemcpyAsync(ctx->b.params, ctx->h_params, sizeof(StepParams) * k_steps, cudaMemcpyHostToDevice, s);
     ks::launch_chunk_init(ctx->b, k_steps, s, true);
-    const std::vector<int> buf = state_turns(ctx, k_steps, src0);
-    const bool aside = refine_aside(ctx);
-    int reader[3] = {-1, -1, -1};  // the last step whose refinement reads the buffer
-    int waited = -1;               // refinements up to this step's are done before the next kernel
-    for (int k = 0; k < k_steps; ++k) {
-        StepArgs a = step_args(ctx, k, k_steps, buf[k], buf[k + 1]);
-        record(ctx, k, 6, capturing);
-        if (ctx->l2_flush_bytes > 0) cudaMemsetAsync(ctx->l2_flush, k & 0xFF, ctx->l2_flush_bytes, s);
-        record(ctx, k, 0, capturing);
-        if (a.hist) cudaMemsetAsync(a.hist, 0, sizeof(unsigned int) * 2 * 8 * 256, s);
-        StepArgs p = a;
-        if (aside) {
-            // The step writes buffer dst and the cell set of two steps ago.
-            a.odd = p.odd = k & 1;
-            const int before = std::max(reader[a.dst], k - 2);
-            if (before > waited) {
-                cudaStreamWaitEvent(s, ctx->ev_refined[before & 3], 0);
-                waited = before;
-                p.overlap = 0;
-            }
-        }
-        ks::launch_propagate(ctx->b, p, s);
-        record(ctx, k, 1, capturing);
-        if (ctx->screening) {
-            if (ks::cells_counted(ctx->b, a)) {
-                record(ctx, k, 2, capturing);
-                ks::launch_count_cells(ctx->b, a, false, s);  // no sort: timed as the cells
-                record(ctx, k, 3, capturing);
-            } else if (ks::sort_cells_fused(ctx->b, a)) {
-                ks::launch_fix_keys(ctx->b, a, s);
-                ks::launch_sort_cells(ctx->b, a, s);  // sort and cells in one launch: timed as the sort
-                record(ctx, k, 2, capturing);
-                record(ctx, k, 3, capturing);
-            } else {
-                ks::launch_fix_keys(ctx->b, a, s);
-                ks::launch_sort(ctx->b, a, s);
-                record(ctx, k, 2, capturing);
-                ks::launch_cells(ctx->b, a, s);
-                record(ctx, k, 3, capturing);
-            }
-            if (aside) {
-                cudaEventRecord(ctx->ev_cells[k & 3], s);
-                cudaStreamWaitEvent(ctx->side, ctx->ev_cells[k & 3], 0);
-                StepArgs r = a;
-                r.overlap = 0;
-                ks::launch_pairs(ctx->b, r, ctx->side);
-                ks::launch_refine(ctx->b, a, ctx->b.conj, ctx->b.conj_cap, ctx->b.chunk, ctx->side);
-                cudaEventRecord(ctx->ev_refined[k & 3], ctx->side);
-                reader[a.src] = reader[a.dst] = k;
-            } else {
+    if (refine_aside(ctx)) {
+        enqueue_aside(ctx, k_steps, src0);
+    } else {
+        int src = src0;
+        for (int k = 0; k < k_steps; ++k) {
+            const StepArgs a = step_args(ctx, k, k_steps, src);
+            record(ctx, k, 6, capturing);
+            if (ctx->l2_flush_bytes > 0) cudaMemsetAsync(ctx->l2_flush, k & 0xFF, ctx->l2_flush_bytes, s);
+            record(ctx, k, 0, capturing);
+            if (a.hist) cudaMemsetAsync(a.hist, 0, sizeof(unsigned int) * 2 * 8 * 256, s);
+            ks::launch_propagate(ctx->b, a, s);
+            record(ctx, k, 1, capturing);
+            if (ctx->screening) {
+                if (ks::cells_counted(ctx->b, a)) {
+                    record(ctx, k, 2, capturing);
+                    ks::launch_count_cells(ctx->b, a, false, s);  // no sort: timed as the cells
+                    record(ctx, k, 3, capturing);
+                } else if (ks::sort_cells_fused(ctx->b, a)) {
+                    ks::launch_fix_keys(ctx->b, a, s);
+                    ks::launch_sort_cells(ctx->b, a, s);  // sort and cells in one launch: timed as the sort
+                    record(ctx, k, 2, capturing);
+                    record(ctx, k, 3, capturing);
+                } else {
+                    ks::launch_fix_keys(ctx->b, a, s);
+                    ks::launch_sort(ctx->b, a, s);
+                    record(ctx, k, 2, capturing);
+                    ks::launch_cells(ctx->b, a, s);
+                    record(ctx, k, 3, capturing);
+                }
                 ks::launch_pairs(ctx->b, a, s);
                 record(ctx, k, 4, capturing);
                 ks::launch_refine(ctx->b, a, ctx->b.conj, ctx->b.conj_cap, ctx->b.chunk, s);
+                if (ctx->dev_sbm) {
+                    ks::launch_step_gate(ctx->b, a, s);
+                    if (ctx->bk.on) ks::launch_sbm_step(ctx->b, a, sbm_args(ctx), s);
+                }
+                record(ctx, k, 5, capturing);
             }
-            if (ctx->dev_sbm) {
-                ks::launch_step_gate(ctx->b, a, s);
-                if (ctx->bk.on) ks::launch_sbm_step(ctx->b, a, sbm_args(ctx), s);
-            }
-            record(ctx, k, 5, capturing);
+            src ^= 1;
         }
     }
-    if (aside) cudaStreamWaitEvent(s, ctx->ev_refined[(k_steps - 1) & 3], 0);
     if (ctx->dev_sbm)
         cudaMemcpyAsync(&ctx->b.chunk->n_live, ctx->b.n_live, sizeof(int), cudaMemcpyDeviceToDevice, s);
     if (ctx->screening)
@@ -1610,8 +1646,12 @@ int ks_create(int device, ks_ctx** out) {
         cudaHostAlloc(&ctx->h_chunk, sizeof(ks::ChunkCtrl), cudaHostAllocDefault) != cudaSuccess)
         rc = KS_ERR_CUDA;
     if (!rc && cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess) rc = KS_ERR_CUDA;
+    if (!rc && (cudaStreamCreateWithFlags(&ctx->ahead, cudaStreamNonBlocking) != cudaSuccess ||
+                cudaEventCreateWithFlags(&ctx->ev_start, cudaEventDisableTiming) != cudaSuccess))
+        rc = KS_ERR_CUDA;
     for (int k = 0; k < 4 && !rc; ++k)
-        if (cudaEventCreateWithFlags(&ctx->ev_cells[k], cudaEventDisableTiming) != cudaSuccess ||
+        if (cudaEventCreateWithFlags(&ctx->ev_prop[k], cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&ctx->ev_cells[k], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ctx->ev_refined[k], cudaEventDisableTiming) != cudaSuccess)
             rc = KS_ERR_CUDA;
     if (!rc) rc = ensure_chunk(ctx, 64);
@@ -1652,7 +1692,10 @@ void ks_destroy(ks_ctx* ctx) {
     if (ctx->h_conj) cudaFreeHost(ctx->h_conj);
     for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->ev_chunk) if (e) cudaEventDestroy(e);
+    if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
+    if (ctx->ahead) cudaStreamDestroy(ctx->ahead);
     for (int k = 0; k < 4; ++k) {
+        if (ctx->ev_prop[k]) cudaEventDestroy(ctx->ev_prop[k]);
         if (ctx->ev_cells[k]) cudaEventDestroy(ctx->ev_cells[k]);
         if (ctx->ev_refined[k]) cudaEventDestroy(ctx->ev_refined[k]);
     }

@@ -114,7 +114,7 @@ struct ChunkCtrl {
     int sort_n;                        // records ordered by the chunk's conjunction sort
 };
 
-// What a step's counted cell build leaves for its tile kernel.
+// What a step's propagation leaves for its counted cell build, and that for its tile kernel.
 struct CellSet {
     float4* sorted32 = nullptr;
     int* sorted_orig = nullptr;
@@ -123,6 +123,8 @@ struct CellSet {
     unsigned long long* hash_keys = nullptr;
     unsigned long long* occ = nullptr;
     int2* survivors = nullptr;
+    unsigned long long* keys = nullptr;    // of the propagation, for this step's cell build
+    float4* rec32 = nullptr;
 };
 
 struct DeviceBuffers {
@@ -246,7 +248,8 @@ struct StepArgs {
     Ctrl* ctrl;                // this step's control block
     Ctrl* ctrl_next;           // next step's control block (speculation outputs)
     int src, dst;              // state buffers holding the start and the end of the step
-    int odd;                   // cells and pairs go to the second set
+    int odd;                   // keys, cells and pairs go to the second set
+    int aside;                 // the propagation runs on another stream than the cell build
     unsigned int* hist;        // radix digit histogram the propagation fills with the keys it emits, or null
     float4* rec32;             // FP32 record of each object, written with its key (object order)
     int overlap;               // the step's kernels may start while their predecessors drain (launch_after)

@@ -3892,7 +3892,7 @@ void launch_seed_ctrl(const DeviceBuffers& b, int n, int src, Ctrl* target, int 
 void launch_propagate(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
     auto go = [&](auto kernel, int grid) {
         launch_after(a.overlap && !a.hist, kernel, grid, a.tune.prop_block, stream, a, b.state[a.src], b.state[a.dst],
-                     b.alive[a.src], b.alive[a.dst], b.keys[0]);
+                     b.alive[a.src], b.alive[a.dst], a.odd ? b.second.keys : b.keys[0]);
     };
     if (a.precision == KS_PRECISION_SPLIT) {
         go(k_propagate_split, grid_for_block(a.n, 5 * kPropBlock / a.tune.prop_block, a.tune.prop_block));
@@ -4173,7 +4173,7 @@ bool cells_counted(const DeviceBuffers& b, const StepArgs& a) {
 namespace {
 CellSet set_of(const DeviceBuffers& b, const StepArgs& a) {
     if (a.odd) return b.second;
-    return CellSet{b.sorted32, b.sorted_orig, b.col_tab, b.items, b.hash_keys, b.occ, b.survivors};
+    return CellSet{b.sorted32, b.sorted_orig, b.col_tab, b.items, b.hash_keys, b.occ, b.survivors, b.keys[0], b.rec32};
 }
 
 // Hash slots of a step's counted build: a power of two above 5/4 of the
@@ -4191,7 +4191,7 @@ int64_t count_slots(const DeviceBuffers& b, int n) {
 void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, cudaStream_t stream) {
     const CellSet set = set_of(b, a);
     CountArgs f{};
-    f.keys = b.keys[0];
+    f.keys = set.keys;
     f.hk = set.hash_keys;
     f.slots = static_cast<unsigned long long>(count_slots(b, a.n));
     f.occ = set.occ;
@@ -4204,13 +4204,13 @@ void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, 
     f.cell_span = reinterpret_cast<int2*>(b.nbr);
     f.sorted_orig = set.sorted_orig;
     f.sorted32 = set.sorted32;
-    f.rec32 = b.rec32;
+    f.rec32 = set.rec32;
     f.col_tab = set.col_tab;
     f.items = set.items;
     f.items_cap = b.items_cap;
     f.per = item_blocks(a.tune, a.n);
     const bool o = a.overlap != 0;
-    launch_after(o && !screen, screen ? k_place<true> : k_place<false>, grid_for(a.n, 8), kBlock, stream, a, f,
+    launch_after(o && !screen && !a.aside, screen ? k_place<true> : k_place<false>, grid_for(a.n, 8), kBlock, stream, a, f,
                  b.state[a.src], b.alive[a.dst]);
     launch_after(o, k_number, grid_for(static_cast<int64_t>(f.slots / 4), 6), kBlock, stream, a, f);
     launch_after(o, k_scatter, grid_for(a.n, 8), kBlock, stream, a, f);

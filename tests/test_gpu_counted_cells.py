@@ -90,3 +90,21 @@ def test_refinement_beside_the_next_step(engine, oracle, ks, spg, chunks):
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
     assert_same_conj(got[2], want[2])
     assert_same_stats(got[3], want[3])
+
+
+def test_refinement_beside_the_next_step_at_larger_sizes(engine, ks):
+    """The sizes at which the propagation shares the cell build's stream and
+    has one of its own again, against the sorted build in one stream."""
+    for n in (140_000, 530_000):
+        st, sz, al = ks.generate_population(n, 20000, n, 40, 7200.0)
+        runs = []
+        try:
+            for form in (2, 1):
+                engine.set_tuning("sort_fused", form)
+                runs.append(run_engine(engine, st, sz, al, 11, spg=4))
+        finally:
+            engine.set_tuning("sort_fused", 2)
+        assert len(runs[0][2]) > 0
+        assert np.array_equal(runs[0][0], runs[1][0]) and np.array_equal(runs[0][1], runs[1][1])
+        assert_same_conj(runs[0][2], runs[1][2])
+        assert_same_stats(runs[0][3], runs[1][3])
