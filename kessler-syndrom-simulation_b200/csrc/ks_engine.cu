@@ -62,6 +62,7 @@ struct ks_ctx {
     int prev = 1;   // state buffer the last step started from
     // Pairs and refinements beside the next step: their stream, and events of cells ready and refinements done (by step, in turn).
     cudaStream_t ahead = nullptr, side = nullptr;
+    char* second_mem = nullptr;   // b.second (but its grown lists), b.state[2], b.alive[2]
     cudaEvent_t ev_start = nullptr, ev_prop[4] = {nullptr, nullptr, nullptr, nullptr},
                 ev_cells[4] = {nullptr, nullptr, nullptr, nullptr}, ev_refined[4] = {nullptr, nullptr, nullptr, nullptr};
     int sort_passes = 8;
@@ -172,16 +173,27 @@ void drop_graphs(ks_ctx* ctx) {
     }
 }
 
+// The second set of what runs beside the next step, in one allocation.
+void free_second(ks_ctx* ctx) {
+    ks::DeviceBuffers& b = ctx->b;
+    dfree(ctx->second_mem);
+    const ks::CellSet grown = b.second;
+    b.second = ks::CellSet{};
+    b.second.items = grown.items;          // grown with the first ones, on their own
+    b.second.survivors = grown.survivors;
+    b.state[2] = nullptr;
+    b.alive[2] = nullptr;
+}
+
 void free_objects(ks_ctx* ctx) {
     ks::DeviceBuffers& b = ctx->b;
-    for (int k = 0; k < 3; ++k) { dfree(b.state[k]); dfree(b.alive[k]); }
+    for (int k = 0; k < 2; ++k) { dfree(b.state[k]); dfree(b.alive[k]); }
     for (int k = 0; k < 2; ++k) { dfree(b.keys[k]); dfree(b.idx[k]); }
     dfree(b.size_m); dfree(b.real_id); dfree(b.ckpt_state); dfree(b.ckpt_alive); dfree(b.block_counts);
     dfree(b.sort_hist); dfree(b.sort_status); dfree(b.sort_ctr);
     dfree(b.cell_begin); dfree(b.cell_key); dfree(b.nbr); dfree(b.cell_len); dfree(b.col_tab); dfree(b.item_part); dfree(b.hash_keys); dfree(b.hash_vals);
     dfree(b.occ);
-    dfree(b.second.sorted32); dfree(b.second.sorted_orig); dfree(b.second.col_tab); dfree(b.second.hash_keys); dfree(b.second.occ);
-    dfree(b.second.keys); dfree(b.second.rec32);
+    free_second(ctx);
     dfree(b.sorted); dfree(b.sorted32); dfree(b.rec32); dfree(b.sorted_orig); dfree(b.fused);
     b.fused_grid = 0;
     dfree(b.n_live); dfree(b.mass_kg); dfree(b.a2m); dfree(b.event_of); dfree(b.coll); dfree(b.sbm_work);
@@ -196,6 +208,8 @@ void free_objects(ks_ctx* ctx) {
     b.sort_status_len = 0;
 }
 
+bool wants_second(ks_ctx* ctx);
+
 int ensure_objects(ks_ctx* ctx, int64_t n) {
     // With fragmentation on the device the arrays are sized once for the
     // population's budget: fragments are appended inside the chunks' graphs.
@@ -206,7 +220,7 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     free_objects(ctx);
     ks::DeviceBuffers& b = ctx->b;
     const int64_t cap = std::max<int64_t>(want, 1024);
-    for (int k = 0; k < (ctx->dev_sbm ? 2 : 3); ++k) {
+    for (int k = 0; k < 2; ++k) {
         KS_CUDA(cudaMalloc(&b.state[k], sizeof(double) * 6 * cap));
         KS_CUDA(cudaMalloc(&b.alive[k], cap));
     }
@@ -240,17 +254,6 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     KS_CUDA(cudaMalloc(&b.sorted32, sizeof(float4) * 2 * cap));
     KS_CUDA(cudaMalloc(&b.rec32, sizeof(float4) * 2 * cap));
     KS_CUDA(cudaMalloc(&b.sorted_orig, sizeof(int) * cap));
-    if (!ctx->dev_sbm) {
-        KS_CUDA(cudaMalloc(&b.second.sorted32, sizeof(float4) * 2 * cap));
-        KS_CUDA(cudaMalloc(&b.second.sorted_orig, sizeof(int) * cap));
-        KS_CUDA(cudaMalloc(&b.second.keys, sizeof(unsigned long long) * cap));
-        KS_CUDA(cudaMalloc(&b.second.rec32, sizeof(float4) * 2 * cap));
-        KS_CUDA(cudaMalloc(&b.second.col_tab, sizeof(int2) * 16 * cap));
-        KS_CUDA(cudaMalloc(&b.second.hash_keys, sizeof(unsigned long long) * h));
-        KS_CUDA(cudaMalloc(&b.second.occ, sizeof(unsigned long long) * (h / 4)));
-        KS_CUDA(cudaMemset(b.second.hash_keys, 0xFF, sizeof(unsigned long long) * h));
-        KS_CUDA(cudaMemset(b.second.occ, 0, sizeof(unsigned long long) * (h / 4)));
-    }
     // Scratch of the fused sort + cell build, sized for this device's grid
     // (looked up here, outside any stream capture).
     if (const int fg = ks::fused_grid()) {
@@ -281,6 +284,39 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     return KS_OK;
 }
 
+// Third state buffer and second set of keys, records, tables and hash: with
+// the first run that uses them (one-shot calls and runs without screening do not).
+int ensure_second(ks_ctx* ctx) {
+    ks::DeviceBuffers& b = ctx->b;
+    if (ctx->second_mem || !wants_second(ctx)) return KS_OK;
+    drop_graphs(ctx);
+    const size_t cap = static_cast<size_t>(b.cap), h = static_cast<size_t>(b.hash_cap);
+    size_t at = 0;
+    auto place = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) / 256 * 256;
+        return o;
+    };
+    const size_t hash = place(8 * h), occ = place(2 * h), state = place(48 * cap), alive = place(cap), keys = place(8 * cap),
+                 rec = place(32 * cap), sorted = place(32 * cap), orig = place(4 * cap), tab = place(128 * cap);
+    KS_CUDA(cudaMalloc(&ctx->second_mem, at));
+    char* m = ctx->second_mem;
+    KS_CUDA(cudaMemsetAsync(m + hash, 0xFF, 8 * h, ctx->stream));
+    KS_CUDA(cudaMemsetAsync(m + occ, 0, 2 * h, ctx->stream));
+    b.second.hash_keys = reinterpret_cast<unsigned long long*>(m + hash);
+    b.second.occ = reinterpret_cast<unsigned long long*>(m + occ);
+    b.state[2] = reinterpret_cast<double*>(m + state);
+    b.alive[2] = reinterpret_cast<uint8_t*>(m + alive);
+    b.second.keys = reinterpret_cast<unsigned long long*>(m + keys);
+    b.second.rec32 = reinterpret_cast<float4*>(m + rec);
+    b.second.sorted32 = reinterpret_cast<float4*>(m + sorted);
+    b.second.sorted_orig = reinterpret_cast<int*>(m + orig);
+    b.second.col_tab = reinterpret_cast<int2*>(m + tab);
+    if (!b.second.survivors) KS_CUDA(cudaMalloc(&b.second.survivors, sizeof(int2) * b.surv_cap));
+    if (!b.second.items) KS_CUDA(cudaMalloc(&b.second.items, sizeof(int4) * b.items_cap));
+    return KS_OK;
+}
+
 int ensure_survivors(ks_ctx* ctx, int64_t want) {
     if (want <= ctx->b.surv_cap) return KS_OK;
     drop_graphs(ctx);
@@ -288,7 +324,7 @@ int ensure_survivors(ks_ctx* ctx, int64_t want) {
     dfree(ctx->b.second.survivors);
     ctx->b.surv_cap = 0;
     KS_CUDA(cudaMalloc(&ctx->b.survivors, sizeof(int2) * want));
-    KS_CUDA(cudaMalloc(&ctx->b.second.survivors, sizeof(int2) * want));
+    if (ctx->second_mem) KS_CUDA(cudaMalloc(&ctx->b.second.survivors, sizeof(int2) * want));
     ctx->b.surv_cap = want;
     return KS_OK;
 }
@@ -300,7 +336,7 @@ int ensure_items(ks_ctx* ctx, int64_t want) {
     dfree(ctx->b.second.items);
     ctx->b.items_cap = 0;
     KS_CUDA(cudaMalloc(&ctx->b.items, sizeof(int4) * want));
-    KS_CUDA(cudaMalloc(&ctx->b.second.items, sizeof(int4) * want));
+    if (ctx->second_mem) KS_CUDA(cudaMalloc(&ctx->b.second.items, sizeof(int4) * want));
     ctx->b.items_cap = want;
     return KS_OK;
 }
@@ -547,10 +583,11 @@ void record_chunk_end(ks_ctx* ctx, bool capturing) {
 // catalogue hour 46.7 / 42.4 / 38.8, at dt 60 s 57.7 / 51.3 / 44.9, 250 000
 // objects 192 / 176 / 160, a million (split) 465 / 450 / 408. (A higher priority for
 // either stream: 250 000 objects 168 -> 186 or 175.)
-bool refine_aside(ks_ctx* ctx) {
-    if (!ctx->screening || ctx->dev_sbm || ctx->profiling || ctx->l2_flush_bytes > 0 || !ctx->b.state[2]) return false;
+bool wants_second(ks_ctx* ctx) {
+    if (!ctx->screening || ctx->dev_sbm || ctx->profiling || ctx->l2_flush_bytes > 0) return false;
     return ks::cells_counted(ctx->b, step_args(ctx, 0, 1, 0));
 }
+bool refine_aside(ks_ctx* ctx) { return ctx->second_mem && wants_second(ctx); }
 
 // State buffers of a chunk's steps: step k from buf[k] to buf[k + 1]. The last
 // one is where two alternating buffers would end, so that a chunk's graph
@@ -999,6 +1036,7 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
     const HostClock::time_point h0 = HostClock::now();
     stash_pending(ctx);  // this chunk's records land in h_conj
     int rc = ensure_chunk(ctx, k_steps);
+    if (!rc) rc = ensure_second(ctx);
     if (rc) return rc;
     double t_end = 0.0;
     fill_params(ctx, k_steps, ctx->t, ctx->steps_done, &t_end);  // uploaded by the chunk itself
@@ -2135,6 +2173,7 @@ int ks_prepare_run(ks_ctx* ctx) {
     if (ctx->steps_per_graph <= 0 || ctx->dev_sbm || plain_run(ctx)) return KS_OK;
     const int k = ctx->steps_per_graph;
     int rc = ensure_chunk(ctx, k);
+    if (!rc) rc = ensure_second(ctx);
     if (!rc) rc = plan_chunk(ctx, k);
     // Both parities: a chunk of an odd number of steps leaves the next one on the other.
     const int cur = ctx->cur;
