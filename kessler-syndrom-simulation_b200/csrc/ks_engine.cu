@@ -2,10 +2,13 @@
 //
 // The device owns the population for the whole run. ks_run advances it in
 // chunks of K steps; a chunk is one CUDA graph (or K direct launches):
-//   chunk_init, then per step: propagate, fix_keys, sort, cells, pairs, refine.
-// The only per-chunk host work is uploading the K rows of lunar positions,
-// reading back K control blocks and the chunk's conjunction records, and
-// ordering those records by (t, i, j). Variable-size outputs live in
+//   chunk_init, then per step: propagate, cells, pairs, refine (a stream each
+//   for propagation, cells, and pairs with refinement; a cell build by sorting
+//   has fix_keys and sort before the cells, in one stream),
+//   then the ordering of the chunk's records by (t, i, j).
+// The only per-chunk host work is uploading the K rows of lunar positions and
+// reading back K control blocks and the chunk's conjunction records. Without
+// screening a launch takes up to 128 steps (run_plain). Variable-size outputs live in
 // fixed-capacity buffers; an overflow flag makes the host grow the buffer,
 // restore the chunk's checkpoint and replay the chunk, so results never
 // depend on capacities (the reference retries its pair list the same way,
@@ -63,6 +66,7 @@ struct ks_ctx {
     // Pairs and refinements beside the next step: their stream, and events of cells ready and refinements done (by step, in turn).
     cudaStream_t ahead = nullptr, side = nullptr;
     char* second_mem = nullptr;   // b.second (but its grown lists), b.state[2], b.alive[2]
+    bool second_denied = false;   // no memory for it: steps stay in one stream
     cudaEvent_t ev_start = nullptr, ev_prop[4] = {nullptr, nullptr, nullptr, nullptr},
                 ev_cells[4] = {nullptr, nullptr, nullptr, nullptr}, ev_refined[4] = {nullptr, nullptr, nullptr, nullptr};
     int sort_passes = 8;
@@ -185,6 +189,16 @@ void free_second(ks_ctx* ctx) {
     b.alive[2] = nullptr;
 }
 
+// Without room for the second set (or for its lists to grow) the steps run in
+// one stream, as they do before it is allocated.
+void deny_second(ks_ctx* ctx) {
+    cudaGetLastError();
+    free_second(ctx);
+    dfree(ctx->b.second.survivors);
+    dfree(ctx->b.second.items);
+    ctx->second_denied = true;
+}
+
 void free_objects(ks_ctx* ctx) {
     ks::DeviceBuffers& b = ctx->b;
     for (int k = 0; k < 2; ++k) { dfree(b.state[k]); dfree(b.alive[k]); }
@@ -194,6 +208,7 @@ void free_objects(ks_ctx* ctx) {
     dfree(b.cell_begin); dfree(b.cell_key); dfree(b.nbr); dfree(b.cell_len); dfree(b.col_tab); dfree(b.item_part); dfree(b.hash_keys); dfree(b.hash_vals);
     dfree(b.occ);
     free_second(ctx);
+    ctx->second_denied = false;
     dfree(b.sorted); dfree(b.sorted32); dfree(b.rec32); dfree(b.sorted_orig); dfree(b.fused);
     b.fused_grid = 0;
     dfree(b.n_live); dfree(b.mass_kg); dfree(b.a2m); dfree(b.event_of); dfree(b.coll); dfree(b.sbm_work);
@@ -288,7 +303,7 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
 // the first run that uses them (one-shot calls and runs without screening do not).
 int ensure_second(ks_ctx* ctx) {
     ks::DeviceBuffers& b = ctx->b;
-    if (ctx->second_mem || !wants_second(ctx)) return KS_OK;
+    if (ctx->second_mem || ctx->second_denied || !wants_second(ctx)) return KS_OK;
     drop_graphs(ctx);
     const size_t cap = static_cast<size_t>(b.cap), h = static_cast<size_t>(b.hash_cap);
     size_t at = 0;
@@ -299,7 +314,12 @@ int ensure_second(ks_ctx* ctx) {
     };
     const size_t hash = place(8 * h), occ = place(2 * h), state = place(48 * cap), alive = place(cap), keys = place(8 * cap),
                  rec = place(32 * cap), sorted = place(32 * cap), orig = place(4 * cap), tab = place(128 * cap);
-    KS_CUDA(cudaMalloc(&ctx->second_mem, at));
+    cudaError_t e = cudaMalloc(&ctx->second_mem, at);
+    if (e == cudaSuccess && !b.second.survivors) e = cudaMalloc(&b.second.survivors, sizeof(int2) * b.surv_cap);
+    if (e == cudaSuccess && !b.second.items) e = cudaMalloc(&b.second.items, sizeof(int4) * b.items_cap);
+    if (e != cudaSuccess) deny_second(ctx);
+    if (e == cudaErrorMemoryAllocation) return KS_OK;
+    KS_CUDA(e);
     char* m = ctx->second_mem;
     KS_CUDA(cudaMemsetAsync(m + hash, 0xFF, 8 * h, ctx->stream));
     KS_CUDA(cudaMemsetAsync(m + occ, 0, 2 * h, ctx->stream));
@@ -312,8 +332,6 @@ int ensure_second(ks_ctx* ctx) {
     b.second.sorted32 = reinterpret_cast<float4*>(m + sorted);
     b.second.sorted_orig = reinterpret_cast<int*>(m + orig);
     b.second.col_tab = reinterpret_cast<int2*>(m + tab);
-    if (!b.second.survivors) KS_CUDA(cudaMalloc(&b.second.survivors, sizeof(int2) * b.surv_cap));
-    if (!b.second.items) KS_CUDA(cudaMalloc(&b.second.items, sizeof(int4) * b.items_cap));
     return KS_OK;
 }
 
@@ -324,7 +342,11 @@ int ensure_survivors(ks_ctx* ctx, int64_t want) {
     dfree(ctx->b.second.survivors);
     ctx->b.surv_cap = 0;
     KS_CUDA(cudaMalloc(&ctx->b.survivors, sizeof(int2) * want));
-    if (ctx->second_mem) KS_CUDA(cudaMalloc(&ctx->b.second.survivors, sizeof(int2) * want));
+    if (ctx->second_mem) {
+        const cudaError_t e = cudaMalloc(&ctx->b.second.survivors, sizeof(int2) * want);
+        if (e == cudaErrorMemoryAllocation) deny_second(ctx);
+        else KS_CUDA(e);
+    }
     ctx->b.surv_cap = want;
     return KS_OK;
 }
@@ -336,7 +358,11 @@ int ensure_items(ks_ctx* ctx, int64_t want) {
     dfree(ctx->b.second.items);
     ctx->b.items_cap = 0;
     KS_CUDA(cudaMalloc(&ctx->b.items, sizeof(int4) * want));
-    if (ctx->second_mem) KS_CUDA(cudaMalloc(&ctx->b.second.items, sizeof(int4) * want));
+    if (ctx->second_mem) {
+        const cudaError_t e = cudaMalloc(&ctx->b.second.items, sizeof(int4) * want);
+        if (e == cudaErrorMemoryAllocation) deny_second(ctx);
+        else KS_CUDA(e);
+    }
     ctx->b.items_cap = want;
     return KS_OK;
 }

@@ -3173,9 +3173,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sort_cells(StepArgs a, Fus
 // many for the cooperative sort's registers) 766 + 1400 us, now 400 + 365.
 // Every launch is bound by the latency of its few dependent L2 accesses at
 // small n and by L2 atomics and random sectors at large n (4-5% of DRAM). With
-// 1M objects in 88 000 cells both builds take about as long (110 against 130
-// us, the tile kernel 220 against 208: objects arrive in a cell in no spatial
-// order).
+// 1M objects in 88 000 cells the builds are closer (104 against 125 us), and
+// the tile kernel takes longer (222 against 208: objects arrive in a cell in no
+// spatial order).
 // ---------------------------------------------------------------------------
 
 // Candidate pairs up to which a cell is screened by its own lanes.
