@@ -658,6 +658,7 @@ void enqueue_aside(ks_ctx* ctx, int k_steps, int src0) {
     for (int k = 0; k < k_steps; ++k) {
         StepArgs a = step_args(ctx, k, k_steps, buf[k], buf[k + 1]);
         a.aside = own;
+        a.beside = 1;
         a.odd = k & 1;
         if (a.odd) a.rec32 = ctx->b.second.rec32;
         StepArgs alone = a;   // for kernels that follow an event of another stream
@@ -1984,7 +1985,7 @@ struct Knobs {
 Knobs current_knobs(const ks_ctx* ctx) {
     return Knobs{ctx->steps_per_graph, ctx->tune.pair_variant, ctx->tune.pair_blocks_per_sm, ctx->tune.subcell_bits,
                  ctx->tune.box_min_rows, static_cast<int>(std::lround(ctx->tune.cell_scale * 1000.0)),
-                 ctx->tune.prop_block, ks::item_blocks(ctx->tune, ctx->n)};
+                 ctx->tune.prop_block, ks::item_blocks(ctx->tune, ctx->n, !ctx->second_mem)};
 }
 
 void put_knobs(ks_ctx* ctx, const Knobs& k, const Ctrl& carry) {

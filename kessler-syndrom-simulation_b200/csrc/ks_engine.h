@@ -250,6 +250,7 @@ struct StepArgs {
     int src, dst;              // state buffers holding the start and the end of the step
     int odd;                   // keys, cells and pairs go to the second set
     int aside;                 // the propagation runs on another stream than the cell build
+    int beside;                // the pairs run beside the next step
     unsigned int* hist;        // radix digit histogram the propagation fills with the keys it emits, or null
     float4* rec32;             // FP32 record of each object, written with its key (object order)
     int overlap;               // the step's kernels may start while their predecessors drain (launch_after)
@@ -341,7 +342,7 @@ void launch_clear_alive(uint8_t* alive, const int64_t* idx, int count, cudaStrea
 void launch_fix_keys(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 void launch_sort(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 bool f32_records(const StepArgs& a);
-int item_blocks(const Tuning& t, int64_t n);  // column blocks per work item for n objects
+int item_blocks(const Tuning& t, int64_t n, bool alone);  // column blocks per work item for n objects
 void launch_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 // Fused sort + cell build: blocks per launch on the current device (0: not
 // available), scratch words for that grid, whether a step takes the fused path.

@@ -3812,10 +3812,14 @@ int fused_digit_bits(const StepArgs& a, int K) {
 // paid less often. Tile kernel, us a step, at 2 / 4 / 8 / 16 / 32 blocks: 33 000
 // objects with a fresh cloud of 5 000 37 / 47 / 63 / 105 / 185; 28 340 at dt 60 s
 // 20 / 21 / 23 / 28 / 28; 250 000 141 / 119 / 112 / 115 / 127; a million 304 / 250 / 225 /
-// 222 / 237; four million 1324 / 1072 / 944 / 886 / 867.
-int item_blocks(const Tuning& t, int64_t n) {
+// 222 / 237, with clouds minutes old - / 276 / 253 / 273 / -; four million 1324 /
+// 1072 / 944 / 886 / 867. Beside the next step (not `alone`) the tail that short
+// items cut off is filled by that step, and their set-up costs it: a million
+// FP64 415 us a step at 8, 405 at 16.
+int item_blocks(const Tuning& t, int64_t n, bool alone) {
     if (t.item_col_blocks > 0) return t.item_col_blocks;
-    return n < (1 << 16) ? 2 : n < (1 << 17) ? 4 : n < (1 << 19) ? 8 : n < (1 << 22) ? 16 : 32;
+    const int64_t eight = alone ? 1 << 20 : 1 << 19;
+    return n < (1 << 16) ? 2 : n < (1 << 17) ? 4 : n < eight ? 8 : n < (1 << 22) ? 16 : 32;
 }
 
 void launch_sort_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream) {
@@ -3842,7 +3846,7 @@ void launch_sort_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t s
     f.col_tab = b.col_tab;
     f.items = b.items;
     f.items_cap = b.items_cap;
-    f.per = item_blocks(a.tune, a.n);
+    f.per = item_blocks(a.tune, a.n, true);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kFusedThreads);
@@ -4170,12 +4174,12 @@ void launch_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream
     // Left empty for the fused launches, which take it so.
     cudaMemsetAsync(b.hash_keys, 0xFF, sizeof(unsigned long long) * b.hash_cap, stream);
     k_items_count<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a.ctrl, b.cell_begin, b.nbr, b.cell_len, b.col_tab, b.item_part,
-                                                           item_blocks(a.tune, a.n));
+                                                           item_blocks(a.tune, a.n, true));
     // Offsets of the heavy, then the light cells' items per chunk of cells, and their total.
     k_scan_small<<<1, 1024, 0, stream>>>(b.item_part, static_cast<int>(2 * ((b.cap + kBlock - 1) / kBlock)),
                                          &a.ctrl->n_items, &a.ctrl->n_cells, 2);
     k_items_write<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a.ctrl, b.cell_begin, b.cell_len, b.item_part, b.items,
-                                                           b.items_cap, item_blocks(a.tune, a.n));
+                                                           b.items_cap, item_blocks(a.tune, a.n, true));
 }
 
 // The counted cell build: packed keys, FP32-gated pair kernels.
@@ -4221,7 +4225,7 @@ void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, 
     f.col_tab = set.col_tab;
     f.items = set.items;
     f.items_cap = b.items_cap;
-    f.per = item_blocks(a.tune, a.n);
+    f.per = item_blocks(a.tune, a.n, !a.beside);
     f.runs = a.n >= (1 << 17);
     const bool o = a.overlap != 0;
     launch_after(o && !screen && !a.aside, screen ? k_place<true> : k_place<false>, grid_for(a.n, 8), kBlock, stream, a, f,
