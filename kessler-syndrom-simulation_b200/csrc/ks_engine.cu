@@ -1998,8 +1998,11 @@ void put_knobs(ks_ctx* ctx, const Knobs& k, const Ctrl& carry) {
     ctx->tune.cell_scale = k.cell_permille / 1000.0;
     ctx->tune.prop_block = k.prop_block;
     ctx->tune.item_col_blocks = k.item_cols;
-    ctx->sort_passes = passes_for_bits(
-        estimate_bits(carry, ctx->dt, ctx->thr, ctx->tune.subcell_bits, ctx->rbits, ctx->tune.cell_scale));
+    const int bits = estimate_bits(carry, ctx->dt, ctx->thr, ctx->tune.subcell_bits, ctx->rbits, ctx->tune.cell_scale);
+    ctx->sort_passes = passes_for_bits(bits);
+    // A trial whose keys are too wide to carry the object index leaves them
+    // unpacked; the next one's may fit again.
+    ctx->pack_keys = ctx->allow_pack && bits + 1 + index_bits(ctx->n) + 2 <= 64;
 }
 
 }  // namespace
