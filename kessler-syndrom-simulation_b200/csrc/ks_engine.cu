@@ -163,6 +163,15 @@ int fail(ks_ctx* c, int code, const std::string& msg) {
         if (e_ != cudaSuccess) return fail(ctx, KS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// A copy that is complete when it returns, ordered in the context's stream:
+// that stream is not ordered after the legacy default one, where an upload
+// from pageable memory may return before it has reached the device.
+int copy_now(ks_ctx* ctx, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
+    KS_CUDA(cudaMemcpyAsync(dst, src, bytes, kind, ctx->stream));
+    KS_CUDA(cudaStreamSynchronize(ctx->stream));
+    return KS_OK;
+}
+
 template <typename T>
 void dfree(T*& p) {
     if (p) cudaFree(p);
@@ -264,7 +273,7 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     KS_CUDA(cudaMalloc(&b.hash_keys, sizeof(unsigned long long) * h));
     KS_CUDA(cudaMalloc(&b.hash_vals, sizeof(int) * h));
     KS_CUDA(cudaMalloc(&b.occ, sizeof(unsigned long long) * (h / 4)));
-    KS_CUDA(cudaMemset(b.occ, 0, sizeof(unsigned long long) * (h / 4)));
+    KS_CUDA(cudaMemsetAsync(b.occ, 0, sizeof(unsigned long long) * (h / 4), ctx->stream));
     KS_CUDA(cudaMalloc(&b.sorted, sizeof(double) * 6 * cap));
     KS_CUDA(cudaMalloc(&b.sorted32, sizeof(float4) * 2 * cap));
     KS_CUDA(cudaMalloc(&b.rec32, sizeof(float4) * 2 * cap));
@@ -276,7 +285,7 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
         b.fused_grid = fg;
     }
     // Every path leaves the cell-key hash empty after a step; it starts so.
-    KS_CUDA(cudaMemset(b.hash_keys, 0xFF, sizeof(unsigned long long) * h));
+    KS_CUDA(cudaMemsetAsync(b.hash_keys, 0xFF, sizeof(unsigned long long) * h, ctx->stream));
     if (ctx->dev_sbm) {
         KS_CUDA(cudaMalloc(&b.n_live, sizeof(int)));
         KS_CUDA(cudaMalloc(&b.mass_kg, sizeof(double) * cap));
@@ -291,7 +300,7 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
         KS_CUDA(cudaMalloc(&b.sbm_next_event, sizeof(int) * 65536));
         KS_CUDA(cudaMalloc(&b.sbm_order, sizeof(int) * b.coll_cap));
         KS_CUDA(cudaMalloc(&b.sbm_first, sizeof(int) * cap));
-        KS_CUDA(cudaMemset(b.sbm_first, 0x7F, sizeof(int) * cap));  // "no event yet"
+        KS_CUDA(cudaMemsetAsync(b.sbm_first, 0x7F, sizeof(int) * cap, ctx->stream));  // "no event yet"
         KS_CUDA(cudaMalloc(&b.sbm_pending, sizeof(int) * 2048));
         KS_CUDA(cudaMalloc(&b.sbm_misc, sizeof(int) * 4));
     }
@@ -429,7 +438,8 @@ int ensure_chunk(ks_ctx* ctx, int k) {
     // Keep the carried speculation across the reallocation.
     Ctrl carry{};
     const bool keep = b.ctrl != nullptr;
-    if (keep) KS_CUDA(cudaMemcpy(&carry, b.ctrl + b.ctrl_len - 2, sizeof(Ctrl), cudaMemcpyDeviceToHost));
+    int rc = KS_OK;
+    if (keep && (rc = copy_now(ctx, &carry, b.ctrl + b.ctrl_len - 2, sizeof(Ctrl), cudaMemcpyDeviceToHost))) return rc;
     dfree(b.ctrl);
     dfree(b.params);
     if (ctx->h_params) cudaFreeHost(ctx->h_params);
@@ -438,11 +448,11 @@ int ensure_chunk(ks_ctx* ctx, int k) {
     ctx->h_ctrl = nullptr;
     b.ctrl_len = k + 2;
     KS_CUDA(cudaMalloc(&b.ctrl, sizeof(Ctrl) * b.ctrl_len));
-    KS_CUDA(cudaMemset(b.ctrl, 0, sizeof(Ctrl) * b.ctrl_len));
+    KS_CUDA(cudaMemsetAsync(b.ctrl, 0, sizeof(Ctrl) * b.ctrl_len, ctx->stream));
     KS_CUDA(cudaMalloc(&b.params, sizeof(StepParams) * k));
     KS_CUDA(cudaHostAlloc(&ctx->h_params, sizeof(StepParams) * k, cudaHostAllocDefault));
     KS_CUDA(cudaHostAlloc(&ctx->h_ctrl, sizeof(Ctrl) * b.ctrl_len, cudaHostAllocDefault));
-    if (keep) KS_CUDA(cudaMemcpy(b.ctrl + b.ctrl_len - 2, &carry, sizeof(Ctrl), cudaMemcpyHostToDevice));
+    if (keep && (rc = copy_now(ctx, b.ctrl + b.ctrl_len - 2, &carry, sizeof(Ctrl), cudaMemcpyHostToDevice))) return rc;
     for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
     ctx->ev.assign(static_cast<size_t>(k) * kPhases, nullptr);
     for (auto& e : ctx->ev) KS_CUDA(cudaEventCreate(&e));
@@ -1812,7 +1822,7 @@ int ks_set_population_batch(ks_ctx* ctx, int32_t realisations, const int64_t* of
     std::vector<uint16_t> rid(static_cast<size_t>(n));
     for (int r = 0; r < realisations; ++r)
         for (int64_t i = offsets[r]; i < offsets[r + 1]; ++i) rid[static_cast<size_t>(i)] = static_cast<uint16_t>(r);
-    if (n > 0) KS_CUDA(cudaMemcpy(ctx->b.real_id, rid.data(), sizeof(uint16_t) * n, cudaMemcpyHostToDevice));
+    if (n > 0 && (rc = copy_now(ctx, ctx->b.real_id, rid.data(), sizeof(uint16_t) * n, cudaMemcpyHostToDevice))) return rc;
     int rbits = 0;
     while ((1 << rbits) < realisations) ++rbits;
     ctx->realisations = realisations;
@@ -2028,7 +2038,7 @@ int ks_autotune(ks_ctx* ctx, int32_t trial_steps, ks_tuning_choice* out) {
     const int sort_passes0 = ctx->sort_passes;
     const Knobs start = current_knobs(ctx);
     Ctrl carry{};
-    KS_CUDA(cudaMemcpy(&carry, carry_slot(ctx), sizeof(Ctrl), cudaMemcpyDeviceToHost));
+    if ((rc = copy_now(ctx, &carry, carry_slot(ctx), sizeof(Ctrl), cudaMemcpyDeviceToHost))) return rc;
     double* snap_state = nullptr;
     uint8_t* snap_alive = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -2300,8 +2310,7 @@ int ks_set_masses(ks_ctx* ctx, int64_t n, const double* mass_kg) {
         return fail(ctx, KS_ERR_ARG, "ks_set_masses: needs one mass per object of the population");
     cudaSetDevice(ctx->device);
     if (ctx->dev_sbm) {
-        if (n > 0) KS_CUDA(cudaMemcpy(ctx->b.mass_kg, mass_kg, sizeof(double) * n, cudaMemcpyHostToDevice));
-        return KS_OK;
+        return n > 0 ? copy_now(ctx, ctx->b.mass_kg, mass_kg, sizeof(double) * n, cudaMemcpyHostToDevice) : KS_OK;
     }
     const int rc = ensure_mirrors(ctx);
     if (rc) return rc;
@@ -2323,9 +2332,10 @@ static int impact_device(ks_ctx* ctx, int64_t target, double projectile_mass_kg,
     KS_CUDA(cudaMemcpyAsync(&rid, b.real_id + target, 2, cudaMemcpyDeviceToHost, ctx->stream));
     KS_CUDA(cudaStreamSynchronize(ctx->stream));
     const int r = ctx->rbits > 0 ? rid : 0;
-    KS_CUDA(cudaMemcpy(&next, b.sbm_next_event + r, sizeof(int), cudaMemcpyDeviceToHost));
+    int rc = copy_now(ctx, &next, b.sbm_next_event + r, sizeof(int), cudaMemcpyDeviceToHost);
+    if (rc) return rc;
     const int id = next++;
-    KS_CUDA(cudaMemcpy(b.sbm_next_event + r, &next, sizeof(int), cudaMemcpyHostToDevice));
+    if ((rc = copy_now(ctx, b.sbm_next_event + r, &next, sizeof(int), cudaMemcpyHostToDevice))) return rc;
     ks::SbmRng side(ctx->bk.seed ^ (0x9E3779B97F4A7C15ull * (static_cast<uint64_t>(r) * 65536u + static_cast<uint64_t>(id) + 1)));
     ks::SbmParent tgt, prj;
     ks::sbm_impact_parents(side, target, s, ks::sbm_mass_or_default(mass), size, projectile_mass_kg, v_rel_km_s, tgt,
@@ -2353,7 +2363,7 @@ static int impact_device(ks_ctx* ctx, int64_t target, double projectile_mass_kg,
     w.realisation = r;
     w.id = id;
     w.record = 0;
-    KS_CUDA(cudaMemcpy(b.sbm_work, &w, sizeof(w), cudaMemcpyHostToDevice));
+    if ((rc = copy_now(ctx, b.sbm_work, &w, sizeof(w), cudaMemcpyHostToDevice))) return rc;
     KS_CUDA(cudaMemsetAsync(&b.chunk->flags, 0, sizeof(int), ctx->stream));
     ks::launch_sbm_prepared(b, sbm_args(ctx), force_consts(), 1, ctx->steps_done, b.state[ctx->cur], b.alive[ctx->cur],
                             carry_slot(ctx), b.chunk, ctx->stream);
@@ -2370,13 +2380,12 @@ static int impact_device(ks_ctx* ctx, int64_t target, double projectile_mass_kg,
     // The real object's fate: destroyed as the SBM projectile or above the
     // catastrophic threshold, else eroded by the ejected mass.
     const uint8_t dead = 0;
-    if (prj.index >= 0) KS_CUDA(cudaMemcpy(b.alive[ctx->cur] + prj.index, &dead, 1, cudaMemcpyHostToDevice));
+    if (prj.index >= 0 && (rc = copy_now(ctx, b.alive[ctx->cur] + prj.index, &dead, 1, cudaMemcpyHostToDevice))) return rc;
     if (tgt.index >= 0) {
-        if (w.catastrophic) KS_CUDA(cudaMemcpy(b.alive[ctx->cur] + tgt.index, &dead, 1, cudaMemcpyHostToDevice));
-        else {
-            const double left = std::max(w.mass[0] - w.budget[0], 0.0);
-            KS_CUDA(cudaMemcpy(b.mass_kg + tgt.index, &left, sizeof(left), cudaMemcpyHostToDevice));
-        }
+        const double left = std::max(w.mass[0] - w.budget[0], 0.0);
+        rc = w.catastrophic ? copy_now(ctx, b.alive[ctx->cur] + tgt.index, &dead, 1, cudaMemcpyHostToDevice)
+                            : copy_now(ctx, b.mass_kg + tgt.index, &left, sizeof(left), cudaMemcpyHostToDevice);
+        if (rc) return rc;
     }
     ctx->n = n_live;
     ctx->bk.out.push_back(ev);
