@@ -143,7 +143,9 @@ int ks_set_l2_flush(ks_ctx* ctx, int64_t bytes);
  * predecessor's unpublished digit counts, or a block of the fused sort makes of
  * a grid barrier, before it gives up; a wait that runs out fails the run with
  * KS_ERR_TIMEOUT and leaves the simulation where the failed chunk of steps
- * began, with no records from it).
+ * began, with no records from it),
+ * "deny_alloc" (0..1000, default 0; for tests: the value-th device allocation
+ * of the context from now on reports that there is no memory, once).
  * Conjunctions, refined and co-orbiting counts and states never change;
  * candidate_pairs and cell_km change with the cell edge. */
 int ks_set_tuning(ks_ctx* ctx, const char* key, int64_t value);

@@ -67,6 +67,7 @@ struct ks_ctx {
     cudaStream_t ahead = nullptr, side = nullptr;
     char* second_mem = nullptr;   // b.second (but its grown lists), b.state[2], b.alive[2]
     bool second_denied = false;   // no memory for it: steps stay in one stream
+    int64_t alloc_deny = 0;       // > 0: the alloc_deny-th device allocation from now reports no memory (tests)
     cudaEvent_t ev_start = nullptr, ev_prop[4] = {nullptr, nullptr, nullptr, nullptr},
                 ev_cells[4] = {nullptr, nullptr, nullptr, nullptr}, ev_refined[4] = {nullptr, nullptr, nullptr, nullptr};
     int sort_passes = 8;
@@ -201,11 +202,33 @@ void free_second(ks_ctx* ctx) {
 // Without room for the second set (or for its lists to grow) the steps run in
 // one stream, as they do before it is allocated.
 void deny_second(ks_ctx* ctx) {
-    cudaGetLastError();
     free_second(ctx);
     dfree(ctx->b.second.survivors);
     dfree(ctx->b.second.items);
     ctx->second_denied = true;
+}
+
+// Device memory for the context. Where there is none left, what the context
+// holds for speed alone is given back before the allocation is tried again: a
+// population that fits without the second set runs, whatever ran before it.
+// (try_alloc: without giving anything back; alloc_deny: a test's countdown to
+// an allocation that reports no memory.)
+template <typename T>
+cudaError_t try_alloc(ks_ctx* ctx, T** p, size_t bytes) {
+    if (ctx->alloc_deny > 0 && --ctx->alloc_deny == 0) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next launch
+    return e;
+}
+
+template <typename T>
+cudaError_t device_alloc(ks_ctx* ctx, T** p, size_t bytes) {
+    const cudaError_t e = try_alloc(ctx, p, bytes);
+    const ks::CellSet& second = ctx->b.second;
+    if (e != cudaErrorMemoryAllocation || !(ctx->second_mem || second.survivors || second.items)) return e;
+    drop_graphs(ctx);
+    deny_second(ctx);
+    return try_alloc(ctx, p, bytes);
 }
 
 void free_objects(ks_ctx* ctx) {
@@ -245,64 +268,72 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     ks::DeviceBuffers& b = ctx->b;
     const int64_t cap = std::max<int64_t>(want, 1024);
     for (int k = 0; k < 2; ++k) {
-        KS_CUDA(cudaMalloc(&b.state[k], sizeof(double) * 6 * cap));
-        KS_CUDA(cudaMalloc(&b.alive[k], cap));
+        KS_CUDA(device_alloc(ctx, &b.state[k], sizeof(double) * 6 * cap));
+        KS_CUDA(device_alloc(ctx, &b.alive[k], cap));
     }
     for (int k = 0; k < 2; ++k) {
-        KS_CUDA(cudaMalloc(&b.keys[k], sizeof(unsigned long long) * cap));
-        KS_CUDA(cudaMalloc(&b.idx[k], sizeof(int) * cap));
+        KS_CUDA(device_alloc(ctx, &b.keys[k], sizeof(unsigned long long) * cap));
+        KS_CUDA(device_alloc(ctx, &b.idx[k], sizeof(int) * cap));
     }
-    KS_CUDA(cudaMalloc(&b.size_m, sizeof(double) * cap));
-    KS_CUDA(cudaMalloc(&b.real_id, sizeof(uint16_t) * cap));
-    KS_CUDA(cudaMalloc(&b.ckpt_state, sizeof(double) * 6 * cap));
-    KS_CUDA(cudaMalloc(&b.ckpt_alive, cap));
+    KS_CUDA(device_alloc(ctx, &b.size_m, sizeof(double) * cap));
+    KS_CUDA(device_alloc(ctx, &b.real_id, sizeof(uint16_t) * cap));
+    KS_CUDA(device_alloc(ctx, &b.ckpt_state, sizeof(double) * 6 * cap));
+    KS_CUDA(device_alloc(ctx, &b.ckpt_alive, cap));
     b.sort_status_len = 8 * 256 * ((cap + 2047) / 2048);
-    KS_CUDA(cudaMalloc(&b.sort_hist, sizeof(unsigned int) * 2 * 8 * 256));  // propagation's counts, then k_fix_keys's
-    KS_CUDA(cudaMalloc(&b.sort_status, sizeof(unsigned int) * b.sort_status_len));
-    KS_CUDA(cudaMalloc(&b.sort_ctr, sizeof(unsigned int) * 8));
-    KS_CUDA(cudaMalloc(&b.block_counts, sizeof(int) * ((cap + 1023) / 1024 + 1)));
-    KS_CUDA(cudaMalloc(&b.cell_begin, sizeof(int) * (cap + 1)));
-    KS_CUDA(cudaMalloc(&b.cell_key, sizeof(unsigned long long) * cap));
-    KS_CUDA(cudaMalloc(&b.nbr, sizeof(int) * 13 * cap));
-    KS_CUDA(cudaMalloc(&b.cell_len, sizeof(int) * cap));
-    KS_CUDA(cudaMalloc(&b.col_tab, sizeof(int2) * 16 * cap));
-    KS_CUDA(cudaMalloc(&b.item_part, sizeof(unsigned int) * 2 * ((cap + 255) / 256 + 1)));
+    KS_CUDA(device_alloc(ctx, &b.sort_hist, sizeof(unsigned int) * 2 * 8 * 256));  // propagation's counts, then k_fix_keys's
+    KS_CUDA(device_alloc(ctx, &b.sort_status, sizeof(unsigned int) * b.sort_status_len));
+    KS_CUDA(device_alloc(ctx, &b.sort_ctr, sizeof(unsigned int) * 8));
+    KS_CUDA(device_alloc(ctx, &b.block_counts, sizeof(int) * ((cap + 1023) / 1024 + 1)));
+    KS_CUDA(device_alloc(ctx, &b.cell_begin, sizeof(int) * (cap + 1)));
+    KS_CUDA(device_alloc(ctx, &b.cell_key, sizeof(unsigned long long) * cap));
+    KS_CUDA(device_alloc(ctx, &b.nbr, sizeof(int) * 13 * cap));
+    KS_CUDA(device_alloc(ctx, &b.cell_len, sizeof(int) * cap));
+    KS_CUDA(device_alloc(ctx, &b.col_tab, sizeof(int2) * 16 * cap));
+    KS_CUDA(device_alloc(ctx, &b.item_part, sizeof(unsigned int) * 2 * ((cap + 255) / 256 + 1)));
     int64_t h = 16;
     while (h < 2 * cap) h <<= 1;
     b.hash_cap = h;
-    KS_CUDA(cudaMalloc(&b.hash_keys, sizeof(unsigned long long) * h));
-    KS_CUDA(cudaMalloc(&b.hash_vals, sizeof(int) * h));
-    KS_CUDA(cudaMalloc(&b.occ, sizeof(unsigned long long) * (h / 4)));
-    KS_CUDA(cudaMemsetAsync(b.occ, 0, sizeof(unsigned long long) * (h / 4), ctx->stream));
-    KS_CUDA(cudaMalloc(&b.sorted, sizeof(double) * 6 * cap));
-    KS_CUDA(cudaMalloc(&b.sorted32, sizeof(float4) * 2 * cap));
-    KS_CUDA(cudaMalloc(&b.rec32, sizeof(float4) * 2 * cap));
-    KS_CUDA(cudaMalloc(&b.sorted_orig, sizeof(int) * cap));
+    KS_CUDA(device_alloc(ctx, &b.hash_keys, sizeof(unsigned long long) * h));
+    KS_CUDA(device_alloc(ctx, &b.hash_vals, sizeof(int) * h));
+    KS_CUDA(device_alloc(ctx, &b.sorted, sizeof(double) * 6 * cap));
+    KS_CUDA(device_alloc(ctx, &b.sorted32, sizeof(float4) * 2 * cap));
+    KS_CUDA(device_alloc(ctx, &b.rec32, sizeof(float4) * 2 * cap));
+    KS_CUDA(device_alloc(ctx, &b.sorted_orig, sizeof(int) * cap));
     // Scratch of the fused sort + cell build, sized for this device's grid
     // (looked up here, outside any stream capture).
     if (const int fg = ks::fused_grid()) {
-        KS_CUDA(cudaMalloc(&b.fused, sizeof(unsigned int) * ks::fused_scratch_words(fg)));
+        KS_CUDA(device_alloc(ctx, &b.fused, sizeof(unsigned int) * ks::fused_scratch_words(fg)));
         b.fused_grid = fg;
     }
     // Every path leaves the cell-key hash empty after a step; it starts so.
     KS_CUDA(cudaMemsetAsync(b.hash_keys, 0xFF, sizeof(unsigned long long) * h, ctx->stream));
     if (ctx->dev_sbm) {
-        KS_CUDA(cudaMalloc(&b.n_live, sizeof(int)));
-        KS_CUDA(cudaMalloc(&b.mass_kg, sizeof(double) * cap));
-        KS_CUDA(cudaMalloc(&b.a2m, sizeof(double) * cap));
-        KS_CUDA(cudaMalloc(&b.event_of, sizeof(int32_t) * cap));
+        KS_CUDA(device_alloc(ctx, &b.n_live, sizeof(int)));
+        KS_CUDA(device_alloc(ctx, &b.mass_kg, sizeof(double) * cap));
+        KS_CUDA(device_alloc(ctx, &b.a2m, sizeof(double) * cap));
+        KS_CUDA(device_alloc(ctx, &b.event_of, sizeof(int32_t) * cap));
         b.coll_cap = ks::kSbmStepEvents;
-        KS_CUDA(cudaMalloc(&b.coll, sizeof(ks::CollisionRec) * b.coll_cap));
-        KS_CUDA(cudaMalloc(&b.sbm_work, sizeof(ks::SbmEventWork) * b.coll_cap));
+        KS_CUDA(device_alloc(ctx, &b.coll, sizeof(ks::CollisionRec) * b.coll_cap));
+        KS_CUDA(device_alloc(ctx, &b.sbm_work, sizeof(ks::SbmEventWork) * b.coll_cap));
         b.sbm_events_cap = kSbmChunkEvents;
-        KS_CUDA(cudaMalloc(&b.sbm_events, sizeof(ks_breakup_event) * b.sbm_events_cap));
+        KS_CUDA(device_alloc(ctx, &b.sbm_events, sizeof(ks_breakup_event) * b.sbm_events_cap));
         KS_CUDA(cudaHostAlloc(&ctx->h_sbm_events, sizeof(ks_breakup_event) * b.sbm_events_cap, cudaHostAllocDefault));
-        KS_CUDA(cudaMalloc(&b.sbm_next_event, sizeof(int) * 65536));
-        KS_CUDA(cudaMalloc(&b.sbm_order, sizeof(int) * b.coll_cap));
-        KS_CUDA(cudaMalloc(&b.sbm_first, sizeof(int) * cap));
+        KS_CUDA(device_alloc(ctx, &b.sbm_next_event, sizeof(int) * 65536));
+        KS_CUDA(device_alloc(ctx, &b.sbm_order, sizeof(int) * b.coll_cap));
+        KS_CUDA(device_alloc(ctx, &b.sbm_first, sizeof(int) * cap));
         KS_CUDA(cudaMemsetAsync(b.sbm_first, 0x7F, sizeof(int) * cap, ctx->stream));  // "no event yet"
-        KS_CUDA(cudaMalloc(&b.sbm_pending, sizeof(int) * 2048));
-        KS_CUDA(cudaMalloc(&b.sbm_misc, sizeof(int) * 4));
+        KS_CUDA(device_alloc(ctx, &b.sbm_pending, sizeof(int) * 2048));
+        KS_CUDA(device_alloc(ctx, &b.sbm_misc, sizeof(int) * 4));
+    }
+    // The counted build's occupancy words come last: a population with room
+    // for all but these sorts its cells.
+    const cudaError_t e = device_alloc(ctx, &b.occ, sizeof(unsigned long long) * (h / 4));
+    if (e == cudaSuccess) {
+        KS_CUDA(cudaMemsetAsync(b.occ, 0, sizeof(unsigned long long) * (h / 4), ctx->stream));
+    } else if (e == cudaErrorMemoryAllocation) {
+        b.occ = nullptr;
+    } else {
+        KS_CUDA(e);
     }
     b.cap = cap;
     return KS_OK;
@@ -323,9 +354,9 @@ int ensure_second(ks_ctx* ctx) {
     };
     const size_t hash = place(8 * h), occ = place(2 * h), state = place(48 * cap), alive = place(cap), keys = place(8 * cap),
                  rec = place(32 * cap), sorted = place(32 * cap), orig = place(4 * cap), tab = place(128 * cap);
-    cudaError_t e = cudaMalloc(&ctx->second_mem, at);
-    if (e == cudaSuccess && !b.second.survivors) e = cudaMalloc(&b.second.survivors, sizeof(int2) * b.surv_cap);
-    if (e == cudaSuccess && !b.second.items) e = cudaMalloc(&b.second.items, sizeof(int4) * b.items_cap);
+    cudaError_t e = try_alloc(ctx, &ctx->second_mem, at);
+    if (e == cudaSuccess && !b.second.survivors) e = try_alloc(ctx, &b.second.survivors, sizeof(int2) * b.surv_cap);
+    if (e == cudaSuccess && !b.second.items) e = try_alloc(ctx, &b.second.items, sizeof(int4) * b.items_cap);
     if (e != cudaSuccess) deny_second(ctx);
     if (e == cudaErrorMemoryAllocation) return KS_OK;
     KS_CUDA(e);
@@ -350,9 +381,9 @@ int ensure_survivors(ks_ctx* ctx, int64_t want) {
     dfree(ctx->b.survivors);
     dfree(ctx->b.second.survivors);
     ctx->b.surv_cap = 0;
-    KS_CUDA(cudaMalloc(&ctx->b.survivors, sizeof(int2) * want));
+    KS_CUDA(device_alloc(ctx, &ctx->b.survivors, sizeof(int2) * want));
     if (ctx->second_mem) {
-        const cudaError_t e = cudaMalloc(&ctx->b.second.survivors, sizeof(int2) * want);
+        const cudaError_t e = try_alloc(ctx, &ctx->b.second.survivors, sizeof(int2) * want);
         if (e == cudaErrorMemoryAllocation) deny_second(ctx);
         else KS_CUDA(e);
     }
@@ -366,9 +397,9 @@ int ensure_items(ks_ctx* ctx, int64_t want) {
     dfree(ctx->b.items);
     dfree(ctx->b.second.items);
     ctx->b.items_cap = 0;
-    KS_CUDA(cudaMalloc(&ctx->b.items, sizeof(int4) * want));
+    KS_CUDA(device_alloc(ctx, &ctx->b.items, sizeof(int4) * want));
     if (ctx->second_mem) {
-        const cudaError_t e = cudaMalloc(&ctx->b.second.items, sizeof(int4) * want);
+        const cudaError_t e = try_alloc(ctx, &ctx->b.second.items, sizeof(int4) * want);
         if (e == cudaErrorMemoryAllocation) deny_second(ctx);
         else KS_CUDA(e);
     }
@@ -410,12 +441,12 @@ int ensure_conj(ks_ctx* ctx, int64_t want) {
         free_conj(ctx);
         ks::DeviceBuffers& b = ctx->b;
         const int64_t tiles = (want + 2047) / 2048;
-        KS_CUDA(cudaMalloc(&b.conj, sizeof(ks_conjunction) * want));
-        KS_CUDA(cudaMalloc(&b.conj_sorted, sizeof(ks_conjunction) * want));
-        for (int k = 0; k < 2; ++k) KS_CUDA(cudaMalloc(&b.conj_keys[k], sizeof(unsigned long long) * want));
-        KS_CUDA(cudaMalloc(&b.conj_status, sizeof(unsigned int) * 256 * 4 * tiles));
-        KS_CUDA(cudaMalloc(&b.conj_hist, sizeof(unsigned int) * 8 * 256));
-        KS_CUDA(cudaMalloc(&b.conj_ctr, sizeof(unsigned int) * 8));
+        KS_CUDA(device_alloc(ctx, &b.conj, sizeof(ks_conjunction) * want));
+        KS_CUDA(device_alloc(ctx, &b.conj_sorted, sizeof(ks_conjunction) * want));
+        for (int k = 0; k < 2; ++k) KS_CUDA(device_alloc(ctx, &b.conj_keys[k], sizeof(unsigned long long) * want));
+        KS_CUDA(device_alloc(ctx, &b.conj_status, sizeof(unsigned int) * 256 * 4 * tiles));
+        KS_CUDA(device_alloc(ctx, &b.conj_hist, sizeof(unsigned int) * 8 * 256));
+        KS_CUDA(device_alloc(ctx, &b.conj_ctr, sizeof(unsigned int) * 8));
         b.conj_cap = want;
     }
     if (want > ctx->h_conj_cap) {
@@ -447,9 +478,9 @@ int ensure_chunk(ks_ctx* ctx, int k) {
     ctx->h_params = nullptr;
     ctx->h_ctrl = nullptr;
     b.ctrl_len = k + 2;
-    KS_CUDA(cudaMalloc(&b.ctrl, sizeof(Ctrl) * b.ctrl_len));
+    KS_CUDA(device_alloc(ctx, &b.ctrl, sizeof(Ctrl) * b.ctrl_len));
     KS_CUDA(cudaMemsetAsync(b.ctrl, 0, sizeof(Ctrl) * b.ctrl_len, ctx->stream));
-    KS_CUDA(cudaMalloc(&b.params, sizeof(StepParams) * k));
+    KS_CUDA(device_alloc(ctx, &b.params, sizeof(StepParams) * k));
     KS_CUDA(cudaHostAlloc(&ctx->h_params, sizeof(StepParams) * k, cudaHostAllocDefault));
     KS_CUDA(cudaHostAlloc(&ctx->h_ctrl, sizeof(Ctrl) * b.ctrl_len, cudaHostAllocDefault));
     if (keep && (rc = copy_now(ctx, b.ctrl + b.ctrl_len - 2, &carry, sizeof(Ctrl), cudaMemcpyHostToDevice))) return rc;
@@ -1242,8 +1273,8 @@ int ensure_plain(ks_ctx* ctx) {
     free_plain(ctx);
     KS_CUDA(cudaHostAlloc(&p.h_params, sizeof(StepParams) * 2 * ks::kManySteps, cudaHostAllocDefault));
     KS_CUDA(cudaHostAlloc(&p.h_counts, sizeof(unsigned int) * 2 * (1 + ks::kManySteps), cudaHostAllocDefault));
-    KS_CUDA(cudaMalloc(&p.d_params, sizeof(StepParams) * 2 * ks::kManySteps));
-    KS_CUDA(cudaMalloc(&p.d_counts, sizeof(unsigned int) * 2 * (1 + ks::kManySteps)));
+    KS_CUDA(device_alloc(ctx, &p.d_params, sizeof(StepParams) * 2 * ks::kManySteps));
+    KS_CUDA(device_alloc(ctx, &p.d_counts, sizeof(unsigned int) * 2 * (1 + ks::kManySteps)));
     for (cudaEvent_t& e : p.done) KS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     return KS_OK;
 }
@@ -1348,7 +1379,7 @@ int ensure_rows(ks_ctx* ctx, int64_t np) {
     ctx->rows_cap = 0;
     KS_CUDA(cudaHostAlloc(&ctx->h_rows, sizeof(double) * 14 * np, cudaHostAllocDefault));
     KS_CUDA(cudaHostAlloc(&ctx->h_pairs, sizeof(int2) * np, cudaHostAllocDefault));
-    KS_CUDA(cudaMalloc(&ctx->d_rows, sizeof(double) * 14 * np));
+    KS_CUDA(device_alloc(ctx, &ctx->d_rows, sizeof(double) * 14 * np));
     ctx->rows_cap = np;
     return KS_OK;
 }
@@ -1442,10 +1473,10 @@ int grow_objects(ks_ctx* ctx, int64_t want) {
     uint8_t* al = nullptr;
     uint16_t* rid = nullptr;
     if (n > 0) {
-        KS_CUDA(cudaMalloc(&st, sizeof(double) * 6 * n));
-        KS_CUDA(cudaMalloc(&sz, sizeof(double) * n));
-        KS_CUDA(cudaMalloc(&al, n));
-        KS_CUDA(cudaMalloc(&rid, sizeof(uint16_t) * n));
+        KS_CUDA(device_alloc(ctx, &st, sizeof(double) * 6 * n));
+        KS_CUDA(device_alloc(ctx, &sz, sizeof(double) * n));
+        KS_CUDA(device_alloc(ctx, &al, n));
+        KS_CUDA(device_alloc(ctx, &rid, sizeof(uint16_t) * n));
         KS_CUDA(cudaMemcpyAsync(st, b.state[ctx->cur], sizeof(double) * 6 * n, cudaMemcpyDeviceToDevice, ctx->stream));
         KS_CUDA(cudaMemcpyAsync(sz, b.size_m, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
         KS_CUDA(cudaMemcpyAsync(al, b.alive[ctx->cur], n, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -1487,7 +1518,7 @@ int ensure_frag_scratch(ks_ctx* ctx, size_t bytes) {
     ctx->frag_scratch = nullptr;
     ctx->frag_scratch_bytes = 0;
     const size_t want = std::max(bytes, size_t(1) << 20);
-    KS_CUDA(cudaMalloc(&ctx->frag_scratch, want));
+    KS_CUDA(device_alloc(ctx, &ctx->frag_scratch, want));
     ctx->frag_scratch_bytes = want;
     return KS_OK;
 }
@@ -1967,6 +1998,10 @@ int ks_set_tuning(ks_ctx* ctx, const char* key, int64_t value) {
         ctx->tune.lookback_polls = static_cast<int>(value);
         drop_graphs(ctx);  // graphs hold the limit in their kernel arguments
     }
+    else if (k == "deny_alloc" && value >= 0 && value <= 1000) {
+        ctx->alloc_deny = value;
+        return KS_OK;
+    }
     else if (k == "pack_keys" && (value == 0 || value == 1)) {
         ctx->allow_pack = value != 0;
         if (ctx->has_pop) {
@@ -2049,8 +2084,8 @@ int ks_autotune(ks_ctx* ctx, int32_t trial_steps, ks_tuning_choice* out) {
         if (e1) cudaEventDestroy(e1);
     };
     if (n > 0) {
-        KS_CUDA(cudaMalloc(&snap_state, sizeof(double) * 6 * n));
-        KS_CUDA(cudaMalloc(&snap_alive, n));
+        KS_CUDA(device_alloc(ctx, &snap_state, sizeof(double) * 6 * n));
+        KS_CUDA(device_alloc(ctx, &snap_alive, n));
         KS_CUDA(cudaMemcpyAsync(snap_state, ctx->b.state[cur0], sizeof(double) * 6 * n, cudaMemcpyDeviceToDevice, ctx->stream));
         KS_CUDA(cudaMemcpyAsync(snap_alive, ctx->b.alive[cur0], n, cudaMemcpyDeviceToDevice, ctx->stream));
     }
@@ -2170,7 +2205,7 @@ int ks_set_l2_flush(ks_ctx* ctx, int64_t bytes) {
     ctx->l2_flush = nullptr;
     ctx->l2_flush_bytes = 0;
     if (bytes > 0) {
-        KS_CUDA(cudaMalloc(&ctx->l2_flush, bytes));
+        KS_CUDA(device_alloc(ctx, &ctx->l2_flush, bytes));
         ctx->l2_flush_bytes = bytes;
     }
     return KS_OK;
