@@ -67,6 +67,8 @@ struct ks_ctx {
     cudaStream_t ahead = nullptr, side = nullptr;
     char* second_mem = nullptr;   // b.second (but its grown lists), b.state[2], b.alive[2]
     bool second_denied = false;   // no memory for it: steps stay in one stream
+    int64_t steps_left = 0;       // of the running call, from the current chunk on
+    int64_t steps_alone = 0;      // run without the second set since the object buffers were made
     int64_t alloc_deny = 0;       // > 0: the alloc_deny-th device allocation from now reports no memory (tests)
     cudaEvent_t ev_start = nullptr, ev_prop[4] = {nullptr, nullptr, nullptr, nullptr},
                 ev_cells[4] = {nullptr, nullptr, nullptr, nullptr}, ev_refined[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -241,6 +243,7 @@ void free_objects(ks_ctx* ctx) {
     dfree(b.occ);
     free_second(ctx);
     ctx->second_denied = false;
+    ctx->steps_alone = 0;
     dfree(b.sorted); dfree(b.sorted32); dfree(b.rec32); dfree(b.sorted_orig); dfree(b.fused);
     b.fused_grid = 0;
     dfree(b.n_live); dfree(b.mass_kg); dfree(b.a2m); dfree(b.event_of); dfree(b.coll); dfree(b.sbm_work);
@@ -339,8 +342,21 @@ int ensure_objects(ks_ctx* ctx, int64_t n) {
     return KS_OK;
 }
 
-// Third state buffer and second set of keys, records, tables and hash: with
-// the first run that uses them (one-shot calls and runs without screening do not).
+// Whether the steps ahead, with those already run in one stream, repay the
+// second set: its allocations take 0.9-1.0 ms whatever their size, and a step
+// gains some 8 us and 6 us more per 100 000 objects (28 340: 12, 250 000: 32, a
+// million: 60-100). Made with the first run whatever its length, it cost a new
+// context's first step 0.25 -> 1.18 ms at 28 340 objects and 0.57 -> 1.64 at a
+// million. A whole graph's chunk makes it in any case: a graph captured without
+// it would be captured again.
+bool second_repays(const ks_ctx* ctx) {
+    const double gain_us = 8.0 + 6e-5 * static_cast<double>(ctx->n);
+    const int64_t steps = std::clamp<int64_t>(static_cast<int64_t>(1000.0 / gain_us), 1, 32);
+    return ctx->steps_left + ctx->steps_alone >= steps;
+}
+
+// Third state buffer and second set of keys, records, tables and hash, where
+// the steps use them (one-shot calls and runs without screening do not).
 int ensure_second(ks_ctx* ctx) {
     ks::DeviceBuffers& b = ctx->b;
     if (ctx->second_mem || ctx->second_denied || !wants_second(ctx)) return KS_OK;
@@ -1104,7 +1120,7 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
     const HostClock::time_point h0 = HostClock::now();
     stash_pending(ctx);  // this chunk's records land in h_conj
     int rc = ensure_chunk(ctx, k_steps);
-    if (!rc) rc = ensure_second(ctx);
+    if (!rc && second_repays(ctx)) rc = ensure_second(ctx);
     if (rc) return rc;
     double t_end = 0.0;
     fill_params(ctx, k_steps, ctx->t, ctx->steps_done, &t_end);  // uploaded by the chunk itself
@@ -1244,6 +1260,7 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
     ctx->steps_done += k_steps;
     ctx->t = t_end;
     ctx->prev = state_turns(ctx, k_steps, ctx->cur)[static_cast<size_t>(k_steps) - 1];
+    if (!ctx->second_mem) ctx->steps_alone += k_steps;
     if (k_steps & 1) ctx->cur ^= 1;
     // Chunk length after collisions: as long as the one that ended early, then
     // doubling back while chunks run through.
@@ -2059,6 +2076,7 @@ int ks_autotune(ks_ctx* ctx, int32_t trial_steps, ks_tuning_choice* out) {
     cudaSetDevice(ctx->device);
     static const int kSpg[] = {8, 16, 32, 64};
     int rc = ensure_chunk(ctx, 64);
+    if (!rc) rc = ensure_second(ctx);  // the trials measure what a long run takes
     if (rc) return rc;
     // Snapshot of everything a trial run changes; restored after every trial
     // and at the end, so tuning leaves the simulation where it was.
@@ -2111,6 +2129,7 @@ int ks_autotune(ks_ctx* ctx, int32_t trial_steps, ks_tuning_choice* out) {
     auto run_steps = [&](int64_t steps) -> int {
         const int64_t end = ctx->steps_done + steps;
         while (ctx->steps_done < end) {
+            ctx->steps_left = end - ctx->steps_done;
             const int chunk = ctx->steps_per_graph > 0 ? ctx->steps_per_graph : 64;
             const int r = run_chunk(ctx, static_cast<int>(std::min<int64_t>(end - ctx->steps_done, chunk)));
             if (r) return r;
@@ -2231,6 +2250,7 @@ int ks_run(ks_ctx* ctx, int64_t steps) {
     while (ctx->steps_done < end) {
         // A chunk may end early, at a step that holds a collision to fragment;
         // while collisions are frequent the chunks stay short (chunk_hint).
+        ctx->steps_left = end - ctx->steps_done;
         const int want = ctx->bk.on && ctx->chunk_hint > 0 ? std::min(chunk, ctx->chunk_hint) : chunk;
         const int k = static_cast<int>(std::min<int64_t>(end - ctx->steps_done, want));
         const HostClock::time_point h0 = HostClock::now();

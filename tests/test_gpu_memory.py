@@ -67,6 +67,27 @@ def test_no_room_for_the_second_set(ks, crowd, nth, spg, chunks):
             assert holds_second(ks, eng) == (nth == 0)
 
 
+@pytest.mark.parametrize("spg", [0, 4])
+def test_short_runs_do_without_the_second_set(ks, crowd, spg):
+    """Its allocation takes longer than a few steps gain by it: a new context
+    does not make it for them, and does once they have added up."""
+    pop, want = crowd
+    with configured(ks, spg) as eng:
+        eng.set_population(*pop)
+        for k in (1, 3):
+            eng.run(k)
+        assert not holds_second(ks, eng)
+        eng.run(8)
+        same(results(eng), want)
+        for _ in range(20):
+            eng.run(1)
+        assert holds_second(ks, eng)
+    with configured(ks, spg) as eng:
+        eng.set_population(*pop)
+        eng.run(32)
+        assert holds_second(ks, eng)
+
+
 @pytest.mark.parametrize("what", ["pairs", "records"])
 @pytest.mark.parametrize("nth", [1, 2])
 @pytest.mark.parametrize("spg", [4, 5])
