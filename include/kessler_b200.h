@@ -105,7 +105,9 @@ int ks_set_l2_flush(ks_ctx* ctx, int64_t bytes);
  * cell-relative records; every variant decides with the exact FP64 filter),
  * "pair_blocks_per_sm" (0 = default: 4 for the split kernel; 5 compiles it for
  * 48 registers),
- * "subcell_bits" (0..3: Morton order of objects inside a cell; default 1), "box_min_rows"
+ * "subcell_bits" (0..3: Morton order of objects inside a cell; default 1; cells
+ * built by counting: in crowded cells of populations above 262 144 objects,
+ * where the steps' candidate pairs repay it), "box_min_rows"
  * (split pair kernel: skip tiles whose row and column blocks are provably
  * apart, for tiles of at least this many rows; default 4; 0 = off), "cell_scale_permille"
  * (1000..4000: grid cell edge = the reference's edge x value/1000),

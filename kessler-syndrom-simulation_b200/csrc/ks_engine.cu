@@ -43,6 +43,7 @@ constexpr int kMaxReplays = 6;
 // the start states (a plain copy of 1 MB takes about 100 us); beyond, one more
 // round trip and a gather of the pairs' rows take less.
 constexpr size_t kLateBytes = size_t(1) << 20;
+constexpr int64_t kOrderObjects = 1 << 18;  // populations whose crowded cells may be put in order (order_pays)
 constexpr int64_t kSbmChunkEvents = 65536;  // breakup records one chunk holds (device fragmentation)
 
 }  // namespace
@@ -98,6 +99,8 @@ struct ks_ctx {
     size_t frag_scratch_bytes = 0;
     bool pack_keys = true;     // object index packed below the cell key in the sort keys
     int64_t max_step_conj = 0; // most conjunction records of one step so far (record buffer sizing)
+    double pairs_each = 0.0;   // candidate pairs per object in the last screened step (0: none yet)
+    bool crowded = false;      // crowded cells are put in order (order_pays)
     bool conj_small = false;   // chunks order their records in one launch (few expected)
     int64_t chunk_spec = 0;    // records a chunk copies back with its control blocks
     int64_t graph_spec[2] = {0, 0};  // the same, as captured in graph_exec[]
@@ -388,6 +391,7 @@ int ensure_second(ks_ctx* ctx) {
     b.second.sorted32 = reinterpret_cast<float4*>(m + sorted);
     b.second.sorted_orig = reinterpret_cast<int*>(m + orig);
     b.second.col_tab = reinterpret_cast<int2*>(m + tab);
+    b.second.crowds = reinterpret_cast<int2*>(b.idx[1]);
     return KS_OK;
 }
 
@@ -602,6 +606,7 @@ StepArgs step_args(ks_ctx* ctx, int k, int k_steps, int src, int dst = -1) {
     a.dst = dst < 0 ? 1 - src : dst;
     a.hist = ctx->screening ? ctx->b.sort_hist : nullptr;  // the propagation counts the sort's digits
     a.rec32 = ctx->b.rec32;
+    a.order = ctx->crowded && ctx->n >= kOrderObjects && ctx->tune.subcell_bits > 0;
     a.pack_bits = ctx->pack_keys ? index_bits(ctx->n) : 0;
     if (ctx->dev_sbm) {
         // Grids sized for the capacity, loops bounded by the live count; the
@@ -948,6 +953,22 @@ int apply_collisions(ks_ctx* ctx, int64_t step, double t0, const std::vector<ks_
 // collision (the chunk is replayed up to that step), and the collisions are
 // fragmented before the next step, as the reference's loop does after each
 // step (src/main.cpp:401-407).
+// Whether the counted build's crowded cells are to be put in sub-cell order
+// (k_order): the launch costs about 5 us a step, and what it saves the tile kernel
+// grows with the candidate pairs an object has. us a step without / with, by pairs
+// per object, one stream: 74 (250 000 objects) 151 / 156, 127 (400 000) 197 / 202,
+// 136 (a million) 363 / 369, 197 (600 000) 262 / 265, 338 (a million) 454 / 449, 432 (two
+// million) 836 / 824, 664 (four) 1900 / 1857, 1078 (600 000) 554 / 504, 1333 (400 000)
+// 460 / 413, 1863 (a million) 1290 / 1110; beside the next step 600 000 with 197:
+// 220 / 230, a million with 338: 392 / 394. Between the two bounds it stays as it
+// is (a change drops the chunk graphs). Below kOrderObjects the gain was smaller (100 000 with 944: 162 / 158) or none
+// (250 000 with 526, clouds just released: 408 / 416). One-shot screening, which
+// knows no step before its own and takes over a millisecond there, orders from
+// that size on.
+bool order_pays(const ks_ctx* ctx) {
+    return ctx->pairs_each >= 600.0 || (ctx->crowded && ctx->pairs_each >= 300.0);
+}
+
 // Sizes the chunk's record buffer and its ordering, and which records come
 // back with the control blocks (shared by both chunk loops).
 int plan_records(ks_ctx* ctx, int k_steps) {
@@ -961,6 +982,10 @@ int plan_records(ks_ctx* ctx, int k_steps) {
         const int64_t span = std::max<int64_t>(k_steps, ctx->steps_per_graph);
         const int64_t want = std::min<int64_t>(ctx->max_step_conj * span * 5 / 4 + 256, int64_t(1) << 30);
         if (want > ctx->b.conj_cap && (rc = ensure_conj(ctx, want))) return rc;
+    }
+    if (ctx->screening && order_pays(ctx) != ctx->crowded) {
+        ctx->crowded = !ctx->crowded;
+        if (ctx->n >= kOrderObjects) drop_graphs(ctx);
     }
     // One-launch ordering of the records where the chunk should hold few.
     const bool small = ctx->screening && ctx->max_step_conj > 0 &&
@@ -1068,6 +1093,7 @@ int run_chunk_dev(ks_ctx* ctx, int k_steps) {
         ctx->timing.candidate_pairs += static_cast<int64_t>(c.candidates);
         ctx->timing.exact_filter_pairs += static_cast<int64_t>(c.exact_evals);
         ctx->timing.refined_pairs += static_cast<int64_t>(c.refined);
+        if (ctx->screening && c.n_alive > 0) ctx->pairs_each = static_cast<double>(c.candidates) / c.n_alive;
     }
     accumulate_timing(ctx, done);
     ctx->timing.steps += done;
@@ -1252,6 +1278,7 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
         ctx->timing.candidate_pairs += static_cast<int64_t>(c.candidates);
         ctx->timing.exact_filter_pairs += static_cast<int64_t>(c.exact_evals);
         ctx->timing.refined_pairs += static_cast<int64_t>(c.refined);
+        if (ctx->screening && c.n_alive > 0) ctx->pairs_each = static_cast<double>(c.candidates) / c.n_alive;
     }
     accumulate_timing(ctx, k_steps);
     ctx->timing.steps += k_steps;
@@ -2736,6 +2763,7 @@ int ks_screen(ks_ctx* ctx, int64_t n, const double* before, const double* after,
         // The counted build keeps a cell's key and count in one word: room for
         // both is known only once the grid is (FLAG_PACK_WIDTH below).
         a.pack_bits = ctx->allow_pack && !wide ? index_bits(n) : 0;
+        a.order = n >= kOrderObjects && ctx->tune.subcell_bits > 0;
         if (ks::cells_counted(ctx->b, a)) {
             ks::launch_count_cells(ctx->b, a, true, ctx->stream);
         } else {

@@ -94,6 +94,7 @@ struct Ctrl {
     unsigned int n_items;              // pair work items (counted build: those at the front of the list)
     unsigned int n_items_back;         // counted build: items at the back of the list
     unsigned int n_tabs;               // counted build: column tables written
+    unsigned int n_crowds;             // counted build: parts of crowded cells to put in order
     unsigned long long placed;         // counted build: objects placed << 32 | cells
     unsigned int item_ticket;          // next pair work item to hand out
     int max_cell;
@@ -125,6 +126,7 @@ struct CellSet {
     int2* survivors = nullptr;
     unsigned long long* keys = nullptr;    // of the propagation, for this step's cell build
     float4* rec32 = nullptr;
+    int2* crowds = nullptr;                // parts of crowded cells (k_order): an array of indices the counted build does not use
 };
 
 struct DeviceBuffers {
@@ -253,6 +255,7 @@ struct StepArgs {
     int beside;                // the pairs run beside the next step
     unsigned int* hist;        // radix digit histogram the propagation fills with the keys it emits, or null
     float4* rec32;             // FP32 record of each object, written with its key (object order)
+    int order;                 // counted build: crowded cells are put in sub-cell order
     int overlap;               // the step's kernels may start while their predecessors drain (launch_after)
     int pack_bits;             // > 0: sort keys carry the object index in their low pack_bits bits
     // Fragmentation on the device (null / 0 otherwise): the live population

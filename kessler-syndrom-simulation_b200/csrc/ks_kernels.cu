@@ -353,7 +353,7 @@ __device__ void ctrl_reset(Ctrl& c) {
     c.vmax_true = 0ull;
     c.candidates = c.co_orbiting = c.refined = c.conj = c.object_steps = c.exact_evals = 0ull;
     c.n_alive = c.n_cells = c.max_cell = c.flags = 0;
-    c.n_items = c.n_items_back = c.n_tabs = 0u;
+    c.n_items = c.n_items_back = c.n_tabs = c.n_crowds = 0u;
     c.placed = 0ull;
     c.item_ticket = 0u;
     c.n_coll = 0u;
@@ -3161,6 +3161,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sort_cells(StepArgs a, Fus
 //   k_number   one pass over the slots: room for each cell's objects (a scan
 //              and one atomic per block), and the list of the cells
 //   k_scatter  the objects' FP32 records to their places
+//   k_order    the objects of crowded cells of large populations to the order
+//              of their sub-cells (before the tile kernel, which alone reads them)
 //   k_cells    a warp per 32 cells: their forward neighbours (occupancy words
 //              say which of the 13 to look up; the lookups are spread over
 //              the lanes); cells with few candidate pairs are screened at
@@ -3190,6 +3192,8 @@ struct CountArgs {
     int shift;                  // fib_slot's shift for the slots' buckets and for the occupancy words
     int2* place;                // per object: its cell's slot (-1: dead), rank in it
     int2* span;                 // per slot: first sorted position and objects of its cell
+    int2* crowds;               // parts of crowded cells to put in order: first position, objects (null: none are)
+    int64_t crowds_cap;
     unsigned long long* cell_key;  // per cell, in no order: its key
     int2* cell_span;            // per cell: as span
     int* sorted_orig;
@@ -3349,12 +3353,24 @@ __global__ void __launch_bounds__(kBlock, kScreen ? 4 : 8) k_place(StepArgs a, C
     }
 }
 
-// Four slots (one bucket) per thread.
+// Cells of more objects are crowded, and are put in order in parts of so many
+// (crowded from 64, 128, 256 or 512 objects on: 600 000 objects in clouds up to
+// an hour old 501 / 501 / 504 / 510 us a step, a million a day old 452 / 448 / 449 / 451).
+constexpr int kCrowded = 256;
+constexpr int kOrderPart = 1024;
+
+// Four slots (one bucket) per thread. kOrder: the crowded cells are listed for k_order.
+template <bool kOrder>
 __global__ void __launch_bounds__(kBlock, 6) k_number(StepArgs a, CountArgs f) {
     after_predecessor();
     Ctrl* ctrl = a.ctrl;
     if (step_void(ctrl)) return;
     __shared__ unsigned long long base_sh;
+    __shared__ unsigned int parts_sh, part_base;
+    if (kOrder) {
+        if (threadIdx.x == 0) parts_sh = 0u;
+        __syncthreads();
+    }
     const int64_t buckets = static_cast<int64_t>(f.slots / 4);
     const unsigned long long cmask = (1ull << f.cbits) - 1;
     unsigned int biggest = 0;
@@ -3362,18 +3378,26 @@ __global__ void __launch_bounds__(kBlock, 6) k_number(StepArgs a, CountArgs f) {
         const int64_t q = blk + threadIdx.x;
         unsigned long long e[4] = {kEmpty, kEmpty, kEmpty, kEmpty};
         if (q < buckets) ld_bucket_cg(f.hk + 4 * q, e);
-        unsigned int k[4], objects = 0, used = 0;
+        unsigned int k[4], objects = 0, used = 0, parts = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             k[j] = e[j] == kEmpty ? 0u : static_cast<unsigned int>(e[j] & cmask);
             objects += k[j];
             used += k[j] > 0;
+            if (kOrder && k[j] > kCrowded) parts += (k[j] + kOrderPart - 1) / kOrderPart;
         }
+        const unsigned int part = kOrder && parts ? atomicAdd(&parts_sh, parts) : 0u;
         // Objects above, cells below: one scan (a block's cells and objects fit 32 bits each).
         unsigned long long total;
         const unsigned long long at = block_exclusive_scan_u64(
             (static_cast<unsigned long long>(objects) << 32) | used, &total);
-        if (threadIdx.x == 0) base_sh = total ? atomicAdd(&ctrl->placed, total) : 0ull;
+        if (threadIdx.x == 0) {
+            base_sh = total ? atomicAdd(&ctrl->placed, total) : 0ull;
+            if (kOrder && parts_sh) {
+                part_base = atomicAdd(&ctrl->n_crowds, parts_sh);
+                parts_sh = 0u;
+            }
+        }
         __syncthreads();
         if (used) {
             unsigned int b0 = static_cast<unsigned int>((base_sh + at) >> 32);
@@ -3387,6 +3411,18 @@ __global__ void __launch_bounds__(kBlock, 6) k_number(StepArgs a, CountArgs f) {
                 f.cell_span[ord++] = sp;
                 b0 += k[j];
                 biggest = max(biggest, k[j]);
+            }
+        }
+        if (kOrder && parts) {
+            int b0 = static_cast<int>((base_sh + at) >> 32);
+            int64_t w = static_cast<int64_t>(part_base) + part;
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j) {
+                const int objects_j = static_cast<int>(j == 0 ? k[0] : j == 1 ? k[1] : j == 2 ? k[2] : k[3]);
+                if (objects_j > kCrowded)
+                    for (int q = 0; q < objects_j; q += kOrderPart, ++w)
+                        if (w < f.crowds_cap) f.crowds[w] = make_int2(b0 + q, min(objects_j - q, kOrderPart));
+                b0 += objects_j;
             }
         }
         __syncthreads();
@@ -3407,6 +3443,67 @@ __global__ void __launch_bounds__(kBlock) k_scatter(StepArgs a, CountArgs f) {
         if (p < 0 || p >= n) continue;
         f.sorted_orig[p] = i;
         st_rec32(f.sorted32 + 2 * static_cast<int64_t>(p), r);
+    }
+}
+
+// Each part of a crowded cell in the Morton order of its objects' sub-cells
+// ("subcell_bits" to an axis), by a counting sort in the block, so that the tile
+// kernel finds blocks of 32 objects whose boxes are apart. Only the order
+// changes: the FP32 positions serve. Bound by latency (loads, shared-memory
+// counts, a scan, stores, 5 us), it runs where the step plan finds the
+// population crowded enough (order_pays). Order of arrival had cost the tile
+// kernel up to a quarter: a step of a million objects in clouds up to an hour
+// old, us, sorted / in order of arrival / in this order: 1083 / 1290 / 1108 in one
+// stream, with the streams of ks_run 1120 (one) / 1172 / 1010.
+__global__ void __launch_bounds__(kBlock) k_order(StepArgs a, const int2* __restrict__ crowds, int64_t crowds_cap,
+                                                  float4* sorted32, int* sorted_orig) {
+    after_predecessor();
+    if (step_void(a.ctrl)) return;
+    constexpr int kEach = kOrderPart / kBlock;
+    __shared__ unsigned int start[2 * kBlock];  // of each code: up to 8^3 codes
+    const int n = live_n(a), sub = a.ctrl->grid.sub, last = (1 << sub) - 1;
+    const float scale = static_cast<float>(1 << sub) / static_cast<float>(a.ctrl->grid.cell);
+    const int parts = static_cast<int>(min(static_cast<int64_t>(a.ctrl->n_crowds), crowds_cap));
+    for (int c = blockIdx.x; c < parts; c += gridDim.x) {
+        const int2 part = crowds[c];
+        if (part.x < 0 || part.x + part.y > n) continue;
+        start[2 * threadIdx.x] = start[2 * threadIdx.x + 1] = 0u;
+        __syncthreads();
+        float4 p[kEach], v[kEach];
+        int orig[kEach];
+        unsigned int code[kEach], rank[kEach];
+#pragma unroll
+        for (int j = 0; j < kEach; ++j) {
+            const int q = j * kBlock + static_cast<int>(threadIdx.x);
+            if (q >= part.y) continue;
+            p[j] = sorted32[2 * static_cast<int64_t>(part.x + q)];
+            v[j] = sorted32[2 * static_cast<int64_t>(part.x + q) + 1];
+            orig[j] = sorted_orig[part.x + q];
+            const unsigned int x = min(max(static_cast<int>(p[j].x * scale), 0), last),
+                               y = min(max(static_cast<int>(p[j].y * scale), 0), last),
+                               z = min(max(static_cast<int>(p[j].z * scale), 0), last);
+            unsigned int m = 0;
+            for (int b = 0; b < sub; ++b)
+                m |= ((x >> b) & 1u) << (3 * b + 2) | ((y >> b) & 1u) << (3 * b + 1) | ((z >> b) & 1u) << (3 * b);
+            code[j] = m;
+            rank[j] = atomicAdd(&start[m], 1u);
+        }
+        __syncthreads();
+        const unsigned int k0 = start[2 * threadIdx.x], k1 = start[2 * threadIdx.x + 1];
+        unsigned int total;
+        const unsigned int at = block_exclusive_scan(k0 + k1, &total);
+        start[2 * threadIdx.x] = at;
+        start[2 * threadIdx.x + 1] = at + k0;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kEach; ++j) {
+            if (j * kBlock + static_cast<int>(threadIdx.x) >= part.y) continue;
+            const int64_t to = part.x + static_cast<int>(start[code[j]] + rank[j]);
+            sorted32[2 * to] = p[j];
+            sorted32[2 * to + 1] = v[j];
+            sorted_orig[to] = orig[j];
+        }
+        __syncthreads();
     }
 }
 
@@ -4190,7 +4287,8 @@ bool cells_counted(const DeviceBuffers& b, const StepArgs& a) {
 namespace {
 CellSet set_of(const DeviceBuffers& b, const StepArgs& a) {
     if (a.odd) return b.second;
-    return CellSet{b.sorted32, b.sorted_orig, b.col_tab, b.items, b.hash_keys, b.occ, b.survivors, b.keys[0], b.rec32};
+    return CellSet{b.sorted32, b.sorted_orig, b.col_tab, b.items, b.hash_keys, b.occ, b.survivors, b.keys[0], b.rec32,
+                   reinterpret_cast<int2*>(b.idx[0])};
 }
 
 // Hash slots of a step's counted build: a power of two above 5/4 of the
@@ -4219,6 +4317,8 @@ void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, 
     f.span = reinterpret_cast<int2*>(b.sorted);
     f.cell_key = b.cell_key;
     f.cell_span = reinterpret_cast<int2*>(b.nbr);
+    f.crowds = a.order ? set.crowds : nullptr;
+    f.crowds_cap = b.cap / 2;
     f.sorted_orig = set.sorted_orig;
     f.sorted32 = set.sorted32;
     f.rec32 = set.rec32;
@@ -4230,7 +4330,7 @@ void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, 
     const bool o = a.overlap != 0;
     launch_after(o && !screen && !a.aside, screen ? k_place<true> : k_place<false>, grid_for(a.n, 8), kBlock, stream, a, f,
                  b.state[a.src], b.alive[a.dst]);
-    launch_after(o, k_number, grid_for(static_cast<int64_t>(f.slots / 4), 6), kBlock, stream, a, f);
+    launch_after(o, f.crowds ? k_number<true> : k_number<false>, grid_for(static_cast<int64_t>(f.slots / 4), 6), kBlock, stream, a, f);
     launch_after(o, k_scatter, grid_for(a.n, 8), kBlock, stream, a, f);
     launch_after(o, k_cells, grid_for_block(4 * static_cast<int64_t>(a.n), kCellBlocksPerSm, kCellBlock), kCellBlock, stream,
                  a, f, b.state[a.src], set.sorted32, set.sorted_orig, set.survivors, b.surv_cap);
@@ -4244,7 +4344,11 @@ void launch_pairs(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream
         // (64; the default: the higher occupancy outweighs a few spilled
         // registers) or for 5 (48; the most its shared memory allows).
         const int bps = a.tune.pair_blocks_per_sm > 0 ? a.tune.pair_blocks_per_sm : 4;
-        launch_after(a.overlap && cells_counted(b, a),
+        const bool order = a.order && cells_counted(b, a);
+        if (order)
+            launch_after(a.overlap != 0, k_order, sm_count() * 4, kBlock, stream, a, set.crowds, b.cap / 2, set.sorted32,
+                         set.sorted_orig);
+        launch_after((a.overlap && cells_counted(b, a)) || (order && a.beside),
                      bps >= 5 ? k_pairs_split<5> : bps == 4 ? k_pairs_split<4> : k_pairs_split<3>, sm_count() * bps, kBlock,
                      stream, a, b.state[a.src], set.sorted32, set.sorted_orig, set.col_tab, set.items, b.items_cap, set.survivors,
                      b.surv_cap, set.hash_keys, set.occ, cells_counted(b, a) ? count_slots(b, a.n) : 0);
