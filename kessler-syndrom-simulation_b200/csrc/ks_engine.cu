@@ -205,8 +205,16 @@ void free_second(ks_ctx* ctx) {
 }
 
 // Without room for the second set (or for its lists to grow) the steps run in
-// one stream, as they do before it is allocated.
+// one stream, as they do before it is allocated. The states that the last step
+// started from, which fragmentation still reads, move out of the third buffer
+// into the one that neither they nor the population occupy.
 void deny_second(ks_ctx* ctx) {
+    ks::DeviceBuffers& b = ctx->b;
+    if (ctx->prev == 2 && b.state[2] && b.state[1 - ctx->cur]) {
+        cudaMemcpyAsync(b.state[1 - ctx->cur], b.state[2], sizeof(double) * 6 * b.cap, cudaMemcpyDeviceToDevice, ctx->stream);
+        cudaStreamSynchronize(ctx->stream);
+        ctx->prev = 1 - ctx->cur;
+    }
     free_second(ctx);
     dfree(ctx->b.second.survivors);
     dfree(ctx->b.second.items);

@@ -161,6 +161,34 @@ def test_fragmentation_without_the_second_set(ks, where, nth, spg):
         assert np.array_equal(stats[f], fx["out_stats"][f]), f
 
 
+@pytest.mark.parametrize("cut", [4, 5, 6, 7, 8])
+def test_second_set_taken_back_between_a_step_and_its_fragmentation(ks, cut):
+    """The first collision's parents are gathered from the step's start and end
+    states into a buffer made then. Where that takes the second set back, the
+    start states stay at hand: chunks of `cut` steps end with them in the third
+    state buffer (5, 6) or in one of the two that remain (4, 7, 8)."""
+    fx = dict(np.load(golden_path("run_breakup.npz")))
+    first = 12   # step of the first collision when nothing is forced before it
+    runs = []
+    for nth in (0, 1):
+        with ks.Engine(0) as eng:
+            eng.set_steps_per_graph(32)
+            eng.set_clock(float(fx["epoch_jd"]), 0.0, float(fx["dt"]))
+            eng.set_screening(True, float(fx["threshold_km"]), float(fx["radius_scale"]), float(fx["min_vrel_km_s"]))
+            eng.set_population(fx["states"], fx["size_m"], fx["alive"])
+            eng.set_masses(fx["mass_kg"])
+            eng.set_breakup(True, float(fx["lc_m"]), 40.0, int(fx["seed"]))
+            eng.prepare_run()
+            eng.run(first + 1 - cut)
+            eng.set_tuning("deny_alloc", nth)
+            eng.run(20)
+            runs.append((*results(eng), eng.take_breakups()))
+    assert runs[0][4]["step"][0] == first and runs[0][4]["fragments"][0] > 0
+    same(runs[1], runs[0])
+    for f in EVENT_FIELDS:
+        assert np.array_equal(runs[1][4][f], runs[0][4][f]), f
+
+
 def test_autotune_and_flush_buffer_take_the_second_set_back(ks, crowd):
     pop, want = crowd
     with configured(ks, 4) as eng:
