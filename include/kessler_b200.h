@@ -158,7 +158,7 @@ typedef struct ks_tuning_choice {
     int32_t pair_variant, pair_blocks_per_sm, subcell_bits, box_min_rows;
     int32_t cell_scale_permille;
     int32_t prop_block;
-    int32_t item_col_blocks;
+    int32_t item_col_blocks;     /* for this population; the rule by the population stays where no trial beat it */
     int32_t trials;              /* configurations timed */
     double ms_per_step_start;    /* device time per step of the starting configuration */
     double ms_per_step_best;     /* ... and of the chosen one */

@@ -2076,13 +2076,18 @@ int ks_set_tuning(ks_ctx* ctx, const char* key, int64_t value) {
 namespace {
 
 struct Knobs {
-    int spg, pair_variant, pair_bps, subcell, box_rows, cell_permille, prop_block, item_cols;
+    int spg, pair_variant, pair_bps, subcell, box_rows, cell_permille, prop_block, item_cols;  // item_cols 0: by the population
 };
+
+// The length of a work item that a configuration gives the population now.
+int item_cols_now(const ks_ctx* ctx, const Knobs& k) {
+    return k.item_cols > 0 ? k.item_cols : ks::item_blocks(ks::Tuning{}, ctx->n, !ctx->second_mem);
+}
 
 Knobs current_knobs(const ks_ctx* ctx) {
     return Knobs{ctx->steps_per_graph, ctx->tune.pair_variant, ctx->tune.pair_blocks_per_sm, ctx->tune.subcell_bits,
                  ctx->tune.box_min_rows, static_cast<int>(std::lround(ctx->tune.cell_scale * 1000.0)),
-                 ctx->tune.prop_block, ks::item_blocks(ctx->tune, ctx->n, !ctx->second_mem)};
+                 ctx->tune.prop_block, ctx->tune.item_col_blocks};
 }
 
 void put_knobs(ks_ctx* ctx, const Knobs& k, const Ctrl& carry) {
@@ -2223,7 +2228,7 @@ int ks_autotune(ks_ctx* ctx, int32_t trial_steps, ks_tuning_choice* out) {
         for (int v : {1000, 1150, 1300, 1500}) if (!rc && v != best.cell_permille) { Knobs c = best; c.cell_permille = v; rc = consider(c); }
     }
     if (ctx->screening)
-        for (int v : {4, 8, 16, 32}) if (!rc && v != best.item_cols) { Knobs c = best; c.item_cols = v; rc = consider(c); }
+        for (int v : {4, 8, 16, 32}) if (!rc && v != item_cols_now(ctx, best)) { Knobs c = best; c.item_cols = v; rc = consider(c); }
     for (int v : {64, 96, 128}) if (!rc && v != best.prop_block) { Knobs c = best; c.prop_block = v; rc = consider(c); }
 
     // Leave the chosen configuration in place and the simulation untouched.
@@ -2243,7 +2248,7 @@ int ks_autotune(ks_ctx* ctx, int32_t trial_steps, ks_tuning_choice* out) {
         out->box_min_rows = best.box_rows;
         out->cell_scale_permille = best.cell_permille;
         out->prop_block = best.prop_block;
-        out->item_col_blocks = best.item_cols;
+        out->item_col_blocks = item_cols_now(ctx, best);
         out->trials = trials;
         out->ms_per_step_start = first_ms;
         out->ms_per_step_best = best_ms;

@@ -1,0 +1,35 @@
+"""What the autotuner leaves in place beside the configuration it chose."""
+import numpy as np
+import pytest
+
+from test_gpu_memory import configured, holds_second
+
+pytestmark = pytest.mark.gpu
+
+
+def test_item_length_by_the_population_outlives_a_tuning_of_another(ks):
+    """A tuning that keeps its starting configuration (here: one that a barrier
+    limit of no polls ends) leaves the length of a work item to the population.
+    The length that 2 000 objects give (2 column blocks) would make 480 000 items
+    of the second population, above the 262 144 the list first holds (126 000 at
+    its own length, 8): the list would grow, and find no memory."""
+    with configured(ks, 4, 20.0) as eng:
+        eng.set_population(*ks.generate_population(3, 2000))
+        eng.set_tuning("sort_fused", 1)
+        eng.set_tuning("lookback_polls", 0)
+        for _ in range(10):   # whether a barrier is found incomplete is a race
+            try:
+                eng.autotune(1)
+            except ks.KsError:
+                break
+            eng.set_tuning("item_col_blocks", 0)
+        else:
+            raise AssertionError("no barrier wait ran out in 10 tunings")
+        eng.set_tuning("lookback_polls", 1 << 22)
+        eng.set_tuning("sort_fused", 2)
+        eng.set_population(*ks.generate_population(17, 28340, 400000, 60, 3600.0))
+        eng.prepare_run()
+        eng.set_buffer_limits(1 << 21, 1 << 18)
+        eng.set_tuning("deny_alloc", 1)
+        eng.run(4)
+        assert holds_second(ks, eng)
