@@ -123,7 +123,8 @@ int ks_set_l2_flush(ks_ctx* ctx, int64_t bytes);
  * flags: 0 row by row over the warp's flagged rows, 1 the default, one pair
  * per lane from a queue when the flags are sparse, 2 always queued),
  * "prop_min_blocks" (4..6, default 4: resident 128-thread blocks per SM the
- * FP64 propagation kernel is compiled for; more blocks, fewer registers each),
+ * FP64 propagation kernel is compiled for; more blocks, fewer registers each;
+ * runs without screening, many steps to a launch, always take 4),
  * "sort_rank_ballot" (radix-sort ranking within a warp: 0, the default, by
  * the hardware match instruction; 1 by eight ballots, one per digit bit),
  * "sort_fused" (2, the default: cells built by counting - every object finds or
@@ -171,7 +172,9 @@ typedef struct ks_tuning_choice {
  * propagation block size, by coordinate descent, and keeps the fastest. Each
  * trial runs at least trial_steps steps (and two graphs). The population,
  * clock, conjunctions and counters are restored afterwards, so the
- * simulation's results are those of an untuned run; only speed changes. */
+ * simulation's results are those of an untuned run; only speed changes.
+ * Without screening the trials run as ks_run does then, many steps to a
+ * launch, and only the propagation block size is tried. */
 int ks_autotune(ks_ctx* ctx, int32_t trial_steps, ks_tuning_choice* out);
 
 /* --- run: Simulation::advance (src/core/orbital.hpp:154) with, per step, the

@@ -1383,7 +1383,7 @@ int run_plain(ks_ctx* ctx, int64_t steps) {
         const int dst = ctx->cur ^ (k & 1);
         ks::launch_propagate_steps(force_consts(), ctx->dt, ctx->precision, static_cast<int>(ctx->n), k, d_rows,
                                    b.state[ctx->cur], b.state[dst], b.alive[ctx->cur], b.alive[dst], d_counts,
-                                   d_counts + 1, ctx->stream);
+                                   d_counts + 1, ctx->tune.prop_block, ctx->stream);
         KS_CUDA(cudaGetLastError());
         KS_CUDA(cudaMemcpyAsync(p.h_counts + slot * kCounts, d_counts, sizeof(unsigned int) * kCounts,
                                 cudaMemcpyDeviceToHost, ctx->stream));
@@ -2167,6 +2167,7 @@ int ks_autotune(ks_ctx* ctx, int32_t trial_steps, ks_tuning_choice* out) {
         return KS_OK;
     };
     auto run_steps = [&](int64_t steps) -> int {
+        if (plain_run(ctx)) return run_plain(ctx, steps);  // as ks_run
         const int64_t end = ctx->steps_done + steps;
         while (ctx->steps_done < end) {
             ctx->steps_left = end - ctx->steps_done;
@@ -2213,7 +2214,8 @@ int ks_autotune(ks_ctx* ctx, int32_t trial_steps, ks_tuning_choice* out) {
         }
         return KS_OK;
     };
-    if (!rc) for (int v : kSpg) if (!rc && v != best.spg) { Knobs c = best; c.spg = v; rc = consider(c); }
+    // Runs without screening launch whole chunks whatever the graph length.
+    if (!rc && !plain_run(ctx)) for (int v : kSpg) if (!rc && v != best.spg) { Knobs c = best; c.spg = v; rc = consider(c); }
     if (ctx->screening) {
         const int pv_bps[][2] = {{1, 0}, {1, 2}, {1, 4}, {0, 0}, {0, 3}, {2, 0}, {2, 3}};
         for (const auto& pb : pv_bps)

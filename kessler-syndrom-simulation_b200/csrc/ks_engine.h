@@ -324,11 +324,12 @@ void launch_seed_ctrl(const DeviceBuffers& b, int n, int src, Ctrl* target, int 
                       cudaStream_t stream);
 void launch_propagate(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 // `steps` (at most kManySteps) steps without screening in one launch, from
-// in / alive_in to out / alive_out (which may be the same buffers).
+// in / alive_in to out / alive_out (which may be the same buffers); block:
+// threads per block (32..128).
 constexpr int kManySteps = 128;
 void launch_propagate_steps(const ForceConsts& fc, double dt, int precision, int n, int steps, const StepParams* sp,
                             const double* in, double* out, const uint8_t* alive_in, uint8_t* alive_out,
-                            unsigned int* alive0, unsigned int* died, cudaStream_t stream);
+                            unsigned int* alive0, unsigned int* died, int block, cudaStream_t stream);
 // Control block of a one-shot screening: reset, then the speed and position
 // bounds of the objects alive after the step at their start-of-step states.
 void launch_screen_init(const DeviceBuffers& b, int n, cudaStream_t stream);

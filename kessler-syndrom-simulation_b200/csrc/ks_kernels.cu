@@ -4023,14 +4023,14 @@ void launch_propagate(const DeviceBuffers& b, const StepArgs& a, cudaStream_t st
 
 void launch_propagate_steps(const ForceConsts& fc, double dt, int precision, int n, int steps, const StepParams* sp,
                             const double* in, double* out, const uint8_t* alive_in, uint8_t* alive_out,
-                            unsigned int* alive0, unsigned int* died, cudaStream_t stream) {
+                            unsigned int* alive0, unsigned int* died, int block, cudaStream_t stream) {
     if (n <= 0) return;
-    const int grid = grid_for_block(n, 4, kPropBlock);
+    const int grid = grid_for_block(n, 4 * kPropBlock / block, block);
     if (precision == KS_PRECISION_SPLIT)
-        k_propagate_steps<true><<<grid, kPropBlock, 0, stream>>>(fc, dt, n, steps, sp, in, out, alive_in, alive_out,
+        k_propagate_steps<true><<<grid, block, 0, stream>>>(fc, dt, n, steps, sp, in, out, alive_in, alive_out,
                                                                  alive0, died);
     else
-        k_propagate_steps<false><<<grid, kPropBlock, 0, stream>>>(fc, dt, n, steps, sp, in, out, alive_in, alive_out,
+        k_propagate_steps<false><<<grid, block, 0, stream>>>(fc, dt, n, steps, sp, in, out, alive_in, alive_out,
                                                                   alive0, died);
 }
 

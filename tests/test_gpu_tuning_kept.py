@@ -33,3 +33,23 @@ def test_item_length_by_the_population_outlives_a_tuning_of_another(ks):
         eng.set_tuning("deny_alloc", 1)
         eng.run(4)
         assert holds_second(ks, eng)
+
+
+@pytest.mark.parametrize("block", [32, 96])
+def test_tuning_without_screening_times_the_steps_a_run_takes(ks, oracle, block):
+    """Without screening a run carries many steps a launch: the graph length says
+    nothing there and is not tried; the threads per block are."""
+    st, sz, al = ks.generate_population(8, 3001)
+    with configured(ks, 0) as eng:
+        eng.set_screening(False)
+        eng.set_tuning("prop_block", block)
+        eng.set_population(st, sz, al)
+        choice = eng.autotune(130)
+        assert choice["trials"] == 1 + sum(v != block for v in (64, 96, 128))
+        assert choice["steps_per_graph"] == 0
+        assert eng.clock() == (0.0, 0) and len(eng.take_step_stats()) == 0
+        eng.set_tuning("prop_block", block)
+        eng.run(140)
+        fs, fa = eng.get_population()
+    want = oracle.run(st, sz, al, steps=140, screen=False)
+    assert np.array_equal(fs, want[0]) and np.array_equal(fa, want[1])
