@@ -50,5 +50,16 @@ def engine(ks):
     eng.close()
 
 
+@pytest.fixture(autouse=True)
+def default_build(request):
+    """The shared engine goes back to the default cell build and item length
+    after each test, whatever the test left: the next one runs what users run."""
+    yield
+    if "engine" in request.fixturenames:
+        eng = request.getfixturevalue("engine")
+        eng.set_tuning("sort_fused", 2)
+        eng.set_tuning("item_col_blocks", 0)
+
+
 def golden_path(name):
     return os.path.join(ROOT, "tests", "golden", name)
