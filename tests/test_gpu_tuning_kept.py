@@ -53,3 +53,22 @@ def test_tuning_without_screening_times_the_steps_a_run_takes(ks, oracle, block)
         fs, fa = eng.get_population()
     want = oracle.run(st, sz, al, steps=140, screen=False)
     assert np.array_equal(fs, want[0]) and np.array_equal(fa, want[1])
+
+
+def test_packed_keys_return_after_a_tuning_trial_too_wide_for_them(ks):
+    """Sub-cell bits tried by the tuner widen the keys past the room for the
+    object index; the configuration it leaves has them packed again and so
+    builds its cells by counting."""
+    st, sz, al = ks.generate_population(31, 5000)   # 15 bits an axis at these cells: no room for a second sub-cell bit
+    with configured(ks, 8, 0.1) as eng:
+        eng.set_screening(True, 2.0, 1.0, 0.01)
+        eng.set_population(st, sz, al)
+        for sub in (2, 1):
+            eng.set_tuning("subcell_bits", sub)
+            eng.run(1)
+            assert (eng.timing()["sort_cells_fused"] == 2) == (sub == 1)
+        choice = eng.autotune(1)
+        assert choice["subcell_bits"] <= 1
+        eng.set_tuning("pair_variant", 2)
+        eng.run(1)
+        assert eng.timing()["sort_cells_fused"] == 2
