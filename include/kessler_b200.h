@@ -130,7 +130,9 @@ int ks_set_l2_flush(ks_ctx* ctx, int64_t bytes);
  * "sort_fused" (2, the default: cells built by counting - every object finds or
  * opens its cell in a hash and takes its place in the cell by its order of
  * arrival, nothing is sorted - wherever the keys carry the object index and the
- * pair kernel gates in FP32; 1: the object sort and the cell build run as one
+ * pair kernel gates in FP32, and sorted as with 1 while the last step held so
+ * many candidate pairs that the sorted order saves the pair kernel more (from
+ * 0.6e9, or 4500 an object, on); 1: the object sort and the cell build run as one
  * cooperative launch of one 1024-thread block per SM, grid barriers between
  * their phases, wherever the keys fit its registers (up to 12 288 per SM) and
  * the keys carry the object index; 0: the separate radix passes and cell

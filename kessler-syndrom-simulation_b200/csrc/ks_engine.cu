@@ -99,7 +99,10 @@ struct ks_ctx {
     size_t frag_scratch_bytes = 0;
     bool pack_keys = true;     // object index packed below the cell key in the sort keys
     int64_t max_step_conj = 0; // most conjunction records of one step so far (record buffer sizing)
-    double pairs_each = 0.0;   // candidate pairs per object in the last screened step (0: none yet)
+    double pairs_each = 0.0;   // candidate pairs per object in the last screened step
+    double step_pairs = 0.0;   // candidate pairs of that step
+    bool pairs_known = false;  // there was such a step
+    bool dense = false;        // cells are built by sorting (sort_pays)
     bool crowded = false;      // crowded cells are put in order (order_pays)
     bool conj_small = false;   // chunks order their records in one launch (few expected)
     int64_t chunk_spec = 0;    // records a chunk copies back with its control blocks
@@ -615,6 +618,7 @@ StepArgs step_args(ks_ctx* ctx, int k, int k_steps, int src, int dst = -1) {
     a.hist = ctx->screening ? ctx->b.sort_hist : nullptr;  // the propagation counts the sort's digits
     a.rec32 = ctx->b.rec32;
     a.order = ctx->crowded && ctx->n >= kOrderObjects && ctx->tune.subcell_bits > 0;
+    a.dense = ctx->dense;
     a.pack_bits = ctx->pack_keys ? index_bits(ctx->n) : 0;
     if (ctx->dev_sbm) {
         // Grids sized for the capacity, loops bounded by the live count; the
@@ -629,8 +633,9 @@ StepArgs step_args(ks_ctx* ctx, int k, int k_steps, int src, int dst = -1) {
         a.pack_bits = ctx->pack_keys ? index_bits(ctx->b.cap) : 0;
     }
     // Kernels of a step start while their predecessors drain, unless events
-    // or flushes lie between them.
-    a.overlap = ctx->profiling == 0 && ctx->l2_flush_bytes == 0;
+    // or flushes lie between them. Not those of dense steps, whose tile kernel
+    // they only hold up (450 000 objects at dt 120 s 3314 us a step, 3267 without).
+    a.overlap = ctx->profiling == 0 && ctx->l2_flush_bytes == 0 && !ctx->dense;
     // The fused sort counts its own digits: the propagation need not.
     if (a.hist && (ks::cells_counted(ctx->b, a) || ks::sort_cells_fused(ctx->b, a))) a.hist = nullptr;
     return a;
@@ -956,11 +961,56 @@ void accumulate_timing(ks_ctx* ctx, int k_steps) {
 
 int apply_collisions(ks_ctx* ctx, int64_t step, double t0, const std::vector<ks_conjunction>& hits);
 
-// Runs one chunk of k_steps; replays it after growing whatever overflowed.
-// With fragmentation on, a chunk ends at the first step that holds a
-// collision (the chunk is replayed up to that step), and the collisions are
-// fragmented before the next step, as the reference's loop does after each
-// step (src/main.cpp:401-407).
+void note_density(ks_ctx* ctx, const Ctrl& c) {
+    ctx->pairs_known = true;
+    ctx->step_pairs = static_cast<double>(c.candidates);
+    if (c.n_alive > 0) ctx->pairs_each = ctx->step_pairs / c.n_alive;
+}
+
+// Whether cells are to be built by sorting, in one stream, although they could
+// be built by counting. The sorted build leaves a cell's objects by sub-cell and
+// then by index, so that the fragments of one cloud, close in place and speed,
+// lie together and the tile kernel skips more blocks; order of arrival scatters
+// them, and k_order sorts parts of 1024 only. The counted build and its streams
+// save 30-100 us a step, that order a share of the tile kernel, which grows with the
+// pairs: us a step counted / sorted, clouds a day old (an hour where marked), with
+// the pairs of a step and per object. Beside the next step: 131 000 objects at dt
+// 120 s (0.75e9, 5689) 596 / 533, 250 000 at 60 s (0.68e9, 2721) 488 / 442 (an hour 468 / 478), at
+// 120 s (2.9e9) 1840 / 1276, 180 000 at 60 s (0.34e9) 284 / 314; ordered by k_order:
+// 300 000 at 60 s (3304) 515 / 541, 450 000 at 60 s (5053) 1020 / 934 (an hour 1087 / 1066), 600 000
+// at 30 s (1491) 546 / 576 and 60 s (6795) 1549 / 1473 (an hour 1666 / 1731), a million at 30 s
+// (2520) 1118 / 1116 and 60 s (11 449) 3758 / 3428. In one stream: 180 000 at 60 s (0.34e9) 314 / 315,
+// 450 000 at 30 s (0.5e9) 390 / 387, 600 000 at 10 s, an hour (0.66e9) 527 / 553, a million
+// at 10 s (0.32e9) 471 / 472 and 20 s (1.06e9) 716 / 660; where the cooperative sort
+// does not fit, two million at 10 s (654) 1081 / 1136 and 20 s (2156) 1919 / 1861.
+bool sort_pays(ks_ctx* ctx, bool streams) {
+    StepArgs a = step_args(ctx, 0, 1, 0);
+    a.dense = 0;
+    if (!ctx->pairs_known || !ks::cells_counted(ctx->b, a)) return false;
+    a.dense = 1;
+    const double keep = ctx->dense ? 0.8 : 1.0;  // a change drops the chunk graphs
+    if (ctx->dev_sbm || ctx->profiling || ctx->l2_flush_bytes > 0) streams = false;
+    if (!streams && !ks::sort_cells_fused(ctx->b, a)) return ctx->pairs_each >= keep * 2000.0;
+    if (!streams) return ctx->step_pairs >= keep * 0.7e9;
+    if (ctx->n < kOrderObjects) return ctx->step_pairs >= keep * 0.6e9;
+    return ctx->pairs_each >= keep * 4500.0;
+}
+
+// The cell build of the steps to come (streams: they have, or are about to get, the second set).
+void plan_build(ks_ctx* ctx, bool streams) {
+    if (!ctx->screening || sort_pays(ctx, streams) == ctx->dense) return;
+    ctx->dense = !ctx->dense;
+    drop_graphs(ctx);
+}
+
+// Whether a run whose density no step has shown yet may be one of those: its
+// first chunk is then a single step. (Pairs of the populations above are at
+// most 4e-11 n^2 cell^3.)
+bool may_be_dense(const ks_ctx* ctx) {
+    const double n = static_cast<double>(ctx->n), cell = 16.0 * ctx->dt + ctx->thr;
+    return ctx->screening && !ctx->pairs_known && n * n * cell * cell * cell >= 1.4e19;
+}
+
 // Whether the counted build's crowded cells are to be put in sub-cell order
 // (k_order): the launch costs about 5 us a step, and what it saves the tile kernel
 // grows with the candidate pairs an object has. us a step without / with, by pairs
@@ -1024,6 +1074,7 @@ int run_chunk_dev(ks_ctx* ctx, int k_steps) {
     if (rc) return rc;
     double t_end = 0.0;
     fill_params(ctx, k_steps, ctx->t, ctx->steps_done, &t_end);
+    plan_build(ctx, false);
     if ((rc = plan_records(ctx, k_steps))) return rc;
     if (ctx->profiling) {
         if ((rc = ensure_graph(ctx, k_steps, true))) return rc;
@@ -1101,7 +1152,7 @@ int run_chunk_dev(ks_ctx* ctx, int k_steps) {
         ctx->timing.candidate_pairs += static_cast<int64_t>(c.candidates);
         ctx->timing.exact_filter_pairs += static_cast<int64_t>(c.exact_evals);
         ctx->timing.refined_pairs += static_cast<int64_t>(c.refined);
-        if (ctx->screening && c.n_alive > 0) ctx->pairs_each = static_cast<double>(c.candidates) / c.n_alive;
+        if (ctx->screening) note_density(ctx, c);
     }
     accumulate_timing(ctx, done);
     ctx->timing.steps += done;
@@ -1149,13 +1200,19 @@ int run_chunk_dev(ks_ctx* ctx, int k_steps) {
 // on the host: the plan of plan_records.
 int plan_chunk(ks_ctx* ctx, int k_steps) { return plan_records(ctx, k_steps); }
 
+// Runs one chunk of k_steps; replays it after growing whatever overflowed.
+// With fragmentation on, a chunk ends at the first step that holds a
+// collision (the chunk is replayed up to that step), and the collisions are
+// fragmented before the next step, as the reference's loop does after each
+// step (src/main.cpp:401-407).
 int run_chunk(ks_ctx* ctx, int k_steps) {
     if (ctx->dev_sbm) return run_chunk_dev(ctx, k_steps);
     const HostClock::time_point h0 = HostClock::now();
     stash_pending(ctx);  // this chunk's records land in h_conj
     int rc = ensure_chunk(ctx, k_steps);
-    if (!rc && second_repays(ctx)) rc = ensure_second(ctx);
     if (rc) return rc;
+    plan_build(ctx, ctx->second_mem || (!ctx->second_denied && second_repays(ctx)));
+    if (second_repays(ctx) && (rc = ensure_second(ctx))) return rc;
     double t_end = 0.0;
     fill_params(ctx, k_steps, ctx->t, ctx->steps_done, &t_end);  // uploaded by the chunk itself
     if ((rc = plan_chunk(ctx, k_steps))) return rc;
@@ -1286,7 +1343,7 @@ int run_chunk(ks_ctx* ctx, int k_steps) {
         ctx->timing.candidate_pairs += static_cast<int64_t>(c.candidates);
         ctx->timing.exact_filter_pairs += static_cast<int64_t>(c.exact_evals);
         ctx->timing.refined_pairs += static_cast<int64_t>(c.refined);
-        if (ctx->screening && c.n_alive > 0) ctx->pairs_each = static_cast<double>(c.candidates) / c.n_alive;
+        if (ctx->screening) note_density(ctx, c);
     }
     accumulate_timing(ctx, k_steps);
     ctx->timing.steps += k_steps;
@@ -1946,7 +2003,10 @@ int64_t ks_population_size(const ks_ctx* ctx) { return ctx ? ctx->n : -1; }
 
 int ks_set_clock(ks_ctx* ctx, double epoch_jd, double t, double dt) {
     if (!ctx || !(dt > 0.0)) return fail(ctx, KS_ERR_ARG, "ks_set_clock: dt must be positive");
-    if (dt != ctx->dt) drop_graphs(ctx);
+    if (dt != ctx->dt) {
+        drop_graphs(ctx);
+        ctx->pairs_known = false;
+    }
     ctx->epoch_jd = epoch_jd;
     ctx->t = t;
     ctx->dt = dt;
@@ -1970,6 +2030,7 @@ int ks_set_screening(ks_ctx* ctx, int enabled, double threshold_km, double radiu
         return fail(ctx, KS_ERR_ARG, "ks_set_screening: bad arguments");
     drop_graphs(ctx);
     ctx->screening = enabled ? 1 : 0;
+    if (threshold_km != ctx->thr) ctx->pairs_known = false;
     ctx->thr = threshold_km;
     ctx->rscale = radius_scale;
     ctx->vmin = min_encounter_speed_km_s;
@@ -2081,7 +2142,7 @@ struct Knobs {
 
 // The length of a work item that a configuration gives the population now.
 int item_cols_now(const ks_ctx* ctx, const Knobs& k) {
-    return k.item_cols > 0 ? k.item_cols : ks::item_blocks(ks::Tuning{}, ctx->n, !ctx->second_mem);
+    return k.item_cols > 0 ? k.item_cols : ks::item_blocks(ks::Tuning{}, ctx->n, !ctx->second_mem, ctx->dense);
 }
 
 Knobs current_knobs(const ks_ctx* ctx) {
@@ -2294,7 +2355,8 @@ int ks_run(ks_ctx* ctx, int64_t steps) {
         // while collisions are frequent the chunks stay short (chunk_hint).
         ctx->steps_left = end - ctx->steps_done;
         const int want = ctx->bk.on && ctx->chunk_hint > 0 ? std::min(chunk, ctx->chunk_hint) : chunk;
-        const int k = static_cast<int>(std::min<int64_t>(end - ctx->steps_done, want));
+        int k = static_cast<int>(std::min<int64_t>(end - ctx->steps_done, want));
+        if (may_be_dense(ctx)) k = 1;
         const HostClock::time_point h0 = HostClock::now();
         rc = run_chunk(ctx, k);
         ctx->timing.host_chunk_ms += host_ms(h0, HostClock::now());
@@ -2310,7 +2372,9 @@ int ks_prepare_run(ks_ctx* ctx) {
     if (ctx->steps_per_graph <= 0 || ctx->dev_sbm || plain_run(ctx)) return KS_OK;
     const int k = ctx->steps_per_graph;
     int rc = ensure_chunk(ctx, k);
-    if (!rc) rc = ensure_second(ctx);
+    if (rc) return rc;
+    plan_build(ctx, !ctx->second_denied);
+    rc = ensure_second(ctx);
     if (!rc) rc = plan_chunk(ctx, k);
     // Both parities: a chunk of an odd number of steps leaves the next one on the other.
     const int cur = ctx->cur;
@@ -2779,6 +2843,7 @@ int ks_screen(ks_ctx* ctx, int64_t n, const double* before, const double* after,
         // both is known only once the grid is (FLAG_PACK_WIDTH below).
         a.pack_bits = ctx->allow_pack && !wide ? index_bits(n) : 0;
         a.order = n >= kOrderObjects && ctx->tune.subcell_bits > 0;
+        a.dense = 0;  // what the steps of a run have shown says nothing of these states
         if (ks::cells_counted(ctx->b, a)) {
             ks::launch_count_cells(ctx->b, a, true, ctx->stream);
         } else {

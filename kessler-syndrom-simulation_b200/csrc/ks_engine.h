@@ -256,6 +256,7 @@ struct StepArgs {
     unsigned int* hist;        // radix digit histogram the propagation fills with the keys it emits, or null
     float4* rec32;             // FP32 record of each object, written with its key (object order)
     int order;                 // counted build: crowded cells are put in sub-cell order
+    int dense;                 // cells are built by sorting although they could be counted
     int overlap;               // the step's kernels may start while their predecessors drain (launch_after)
     int pack_bits;             // > 0: sort keys carry the object index in their low pack_bits bits
     // Fragmentation on the device (null / 0 otherwise): the live population
@@ -346,7 +347,7 @@ void launch_clear_alive(uint8_t* alive, const int64_t* idx, int count, cudaStrea
 void launch_fix_keys(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 void launch_sort(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 bool f32_records(const StepArgs& a);
-int item_blocks(const Tuning& t, int64_t n, bool alone);  // column blocks per work item for n objects
+int item_blocks(const Tuning& t, int64_t n, bool alone, bool dense = false);  // column blocks per work item for n objects
 void launch_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream);
 // Fused sort + cell build: blocks per launch on the current device (0: not
 // available), scratch words for that grid, whether a step takes the fused path.

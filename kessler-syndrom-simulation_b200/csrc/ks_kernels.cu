@@ -3912,9 +3912,13 @@ int fused_digit_bits(const StepArgs& a, int K) {
 // 222 / 237, with clouds minutes old - / 276 / 253 / 273 / -; four million 1324 /
 // 1072 / 944 / 886 / 867. Beside the next step (not `alone`) the tail that short
 // items cut off is filled by that step, and their set-up costs it: a million
-// FP64 415 us a step at 8, 405 at 16.
-int item_blocks(const Tuning& t, int64_t n, bool alone) {
+// FP64 415 us a step at 8, 405 at 16. Dense populations, whose cells are sorted
+// (sort_pays), fill the chip at any size; build and tile kernel at 4 / 8 / 16 / 32 / 64:
+// 131 000 objects at dt 120 s 548 / 503 / 524 / 508 / 504, 250 000 1511 / 1277 / 1199 / 1272 / 1253,
+// 450 000 at 60 s 1085 / 923 / 850 / 842 / 913, a million 4211 / 3526 / 3183 / 3028 / 2983.
+int item_blocks(const Tuning& t, int64_t n, bool alone, bool dense) {
     if (t.item_col_blocks > 0) return t.item_col_blocks;
+    if (dense) return 16;
     const int64_t eight = alone ? 1 << 20 : 1 << 19;
     return n < (1 << 16) ? 2 : n < (1 << 17) ? 4 : n < eight ? 8 : n < (1 << 22) ? 16 : 32;
 }
@@ -3943,7 +3947,7 @@ void launch_sort_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t s
     f.col_tab = b.col_tab;
     f.items = b.items;
     f.items_cap = b.items_cap;
-    f.per = item_blocks(a.tune, a.n, true);
+    f.per = item_blocks(a.tune, a.n, true, a.dense != 0);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kFusedThreads);
@@ -4271,17 +4275,17 @@ void launch_cells(const DeviceBuffers& b, const StepArgs& a, cudaStream_t stream
     // Left empty for the fused launches, which take it so.
     cudaMemsetAsync(b.hash_keys, 0xFF, sizeof(unsigned long long) * b.hash_cap, stream);
     k_items_count<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a.ctrl, b.cell_begin, b.nbr, b.cell_len, b.col_tab, b.item_part,
-                                                           item_blocks(a.tune, a.n, true));
+                                                           item_blocks(a.tune, a.n, true, a.dense != 0));
     // Offsets of the heavy, then the light cells' items per chunk of cells, and their total.
     k_scan_small<<<1, 1024, 0, stream>>>(b.item_part, static_cast<int>(2 * ((b.cap + kBlock - 1) / kBlock)),
                                          &a.ctrl->n_items, &a.ctrl->n_cells, 2);
     k_items_write<<<grid_for(a.n, 8), kBlock, 0, stream>>>(a.ctrl, b.cell_begin, b.cell_len, b.item_part, b.items,
-                                                           b.items_cap, item_blocks(a.tune, a.n, true));
+                                                           b.items_cap, item_blocks(a.tune, a.n, true, a.dense != 0));
 }
 
 // The counted cell build: packed keys, FP32-gated pair kernels.
 bool cells_counted(const DeviceBuffers& b, const StepArgs& a) {
-    return a.tune.sort_fused == 2 && b.occ && a.pack_bits > 0 && a.n > 0 && f32_records(a);
+    return a.tune.sort_fused == 2 && !a.dense && b.occ && a.pack_bits > 0 && a.n > 0 && f32_records(a);
 }
 
 namespace {
