@@ -101,8 +101,10 @@ struct ks_ctx {
     int64_t max_step_conj = 0; // most conjunction records of one step so far (record buffer sizing)
     double pairs_each = 0.0;   // candidate pairs per object in the last screened step
     double step_pairs = 0.0;   // candidate pairs of that step
+    double refined_each = 0.0; // and refined pairs per object
     bool pairs_known = false;  // there was such a step
     bool dense = false;        // cells are built by sorting (sort_pays)
+    bool one_stream = false;   // refinement outweighs the rest (plan_build)
     bool crowded = false;      // crowded cells are put in order (order_pays)
     bool conj_small = false;   // chunks order their records in one launch (few expected)
     int64_t chunk_spec = 0;    // records a chunk copies back with its control blocks
@@ -685,7 +687,7 @@ void record_chunk_end(ks_ctx* ctx, bool capturing) {
 // objects 192 / 176 / 160, a million (split) 465 / 450 / 408. (A higher priority for
 // either stream: 250 000 objects 168 -> 186 or 175.)
 bool wants_second(ks_ctx* ctx) {
-    if (!ctx->screening || ctx->dev_sbm || ctx->profiling || ctx->l2_flush_bytes > 0) return false;
+    if (!ctx->screening || ctx->dev_sbm || ctx->profiling || ctx->l2_flush_bytes > 0 || ctx->one_stream) return false;
     return ks::cells_counted(ctx->b, step_args(ctx, 0, 1, 0));
 }
 bool refine_aside(ks_ctx* ctx) { return ctx->second_mem && wants_second(ctx); }
@@ -964,7 +966,10 @@ int apply_collisions(ks_ctx* ctx, int64_t step, double t0, const std::vector<ks_
 void note_density(ks_ctx* ctx, const Ctrl& c) {
     ctx->pairs_known = true;
     ctx->step_pairs = static_cast<double>(c.candidates);
-    if (c.n_alive > 0) ctx->pairs_each = ctx->step_pairs / c.n_alive;
+    if (c.n_alive > 0) {
+        ctx->pairs_each = ctx->step_pairs / c.n_alive;
+        ctx->refined_each = static_cast<double>(c.refined) / c.n_alive;
+    }
 }
 
 // Whether cells are to be built by sorting, in one stream, although they could
@@ -996,11 +1001,20 @@ bool sort_pays(ks_ctx* ctx, bool streams) {
     return ctx->pairs_each >= keep * 4500.0;
 }
 
-// The cell build of the steps to come (streams: they have, or are about to get, the second set).
+// The streams and the cell build of the steps to come (streams: they have, or
+// are about to get, the second set). Where refinement outweighs the rest, steps
+// run in one stream: beside another step's kernels it shares the L1 cache
+// with their shared memory (refine). us a step, beside / in one stream, by refined pairs per
+// object: 8 (600 000 objects) 1925 / 1907, 14 (a million) 6275 / 6534, 18 (100 000) 691 / 680, 30 (250 000)
+// 1999 / 2046, 70 (60 000) 1451 / 1158, 138 (100 000) 3866 / 3231, 222 (60 000) 4240 / 3316.
 void plan_build(ks_ctx* ctx, bool streams) {
-    if (!ctx->screening || sort_pays(ctx, streams) == ctx->dense) return;
-    ctx->dense = !ctx->dense;
-    drop_graphs(ctx);
+    if (!ctx->screening) return;
+    const bool one = ctx->pairs_known && ctx->refined_each >= (ctx->one_stream ? 32.0 : 40.0);
+    const bool dense = sort_pays(ctx, streams && !one);
+    if (one == ctx->one_stream && dense == ctx->dense) return;
+    ctx->one_stream = one;
+    ctx->dense = dense;
+    drop_graphs(ctx);  // they hold both
 }
 
 // Whether a run whose density no step has shown yet may be one of those: its
