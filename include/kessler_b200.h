@@ -113,7 +113,8 @@ int ks_set_l2_flush(ks_ctx* ctx, int64_t bytes);
  * (1000..4000: grid cell edge = the reference's edge x value/1000),
  * "prop_block" (32..128, threads per block of the propagation kernels),
  * "item_col_blocks" (1..64, column blocks of 32 per pair-kernel work item; 0,
- * the default: by the population, 2 below 65 536 objects to 32 above 4M),
+ * the default: by the population, 2 below 65 536 objects to 32 above 4M, up to
+ * 16 below 131 072 where a few cells hold most of its pairs),
  * "pack_keys" (1: the radix sort carries the object index in the low bits of
  * its keys where they leave room, the default; 0: a separate index array),
  * "pair_gate_x2" (1, the default: the FP32 pair gate evaluates two rows per

@@ -95,6 +95,7 @@ struct Ctrl {
     unsigned int n_items_back;         // counted build: items at the back of the list
     unsigned int n_tabs;               // counted build: column tables written
     unsigned int n_crowds;             // counted build: parts of crowded cells to put in order
+    unsigned long long crowd_pairs;    // counted build: pairs inside crowded cells, about
     unsigned long long placed;         // counted build: objects placed << 32 | cells
     unsigned int item_ticket;          // next pair work item to hand out
     int max_cell;

@@ -354,7 +354,7 @@ __device__ void ctrl_reset(Ctrl& c) {
     c.candidates = c.co_orbiting = c.refined = c.conj = c.object_steps = c.exact_evals = 0ull;
     c.n_alive = c.n_cells = c.max_cell = c.flags = 0;
     c.n_items = c.n_items_back = c.n_tabs = c.n_crowds = 0u;
-    c.placed = 0ull;
+    c.placed = c.crowd_pairs = 0ull;
     c.item_ticket = 0u;
     c.n_coll = 0u;
     c.grid = GridParams{};
@@ -3204,6 +3204,7 @@ struct CountArgs {
     int4* items;
     int64_t items_cap;
     int per;
+    int lift;                   // per may grow with crowd_pairs (lifted_per)
     int runs;                   // z runs of cells share neighbouring buckets (home_bucket)
 };
 
@@ -3375,6 +3376,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_number(StepArgs a, CountArgs f) {
     const int64_t buckets = static_cast<int64_t>(f.slots / 4);
     const unsigned long long cmask = (1ull << f.cbits) - 1;
     unsigned int biggest = 0;
+    unsigned long long crowd = 0;
     for (int64_t blk = static_cast<int64_t>(blockIdx.x) * kBlock; blk < buckets; blk += static_cast<int64_t>(gridDim.x) * kBlock) {
         const int64_t q = blk + threadIdx.x;
         unsigned long long e[4] = {kEmpty, kEmpty, kEmpty, kEmpty};
@@ -3412,6 +3414,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_number(StepArgs a, CountArgs f) {
                 f.cell_span[ord++] = sp;
                 b0 += k[j];
                 biggest = max(biggest, k[j]);
+                if (k[j] > kCrowded) crowd += static_cast<unsigned long long>(k[j]) * k[j] / 2;
             }
         }
         if (kOrder && parts) {
@@ -3429,7 +3432,9 @@ __global__ void __launch_bounds__(kBlock, 6) k_number(StepArgs a, CountArgs f) {
         __syncthreads();
     }
     biggest = warp_max(biggest);
+    crowd = warp_sum(crowd);
     if ((threadIdx.x & 31) == 0 && biggest > 0) atomicMax(&ctrl->max_cell, static_cast<int>(biggest));
+    if ((threadIdx.x & 31) == 0 && crowd > 0) atomicAdd(&ctrl->crowd_pairs, crowd);
 }
 
 __global__ void __launch_bounds__(kBlock) k_scatter(StepArgs a, CountArgs f) {
@@ -3557,6 +3562,16 @@ __device__ __forceinline__ unsigned occ_three(const CountArgs& f, unsigned long 
     return static_cast<unsigned>(w >> ((key & 31) + 15)) & 7u;
 }
 
+// Column blocks of a work item (item_blocks) in a small population a few of
+// whose cells hold most of its pairs: items short enough to spread one crowded
+// cell over the chip are too many where that cell is a whole cloud. us a step
+// at 2 / 4 / 8 / 16 blocks, 60 000 objects, by pairs inside crowded cells: 15M (an hour
+// after release) 92 / 77 / 71 / 82, 20M (40 000 objects, a minute) 70 / 59 / 65 / 73, 110M (ten
+// minutes) 227 / 181 / 154 / 143, 150M (a minute) 271 / 222 / 194 / 182, 240M (in one cloud) 837 / 588 / 454 / 385.
+__device__ __forceinline__ int lifted_per(int per, unsigned long long crowd_pairs) {
+    return max(per, crowd_pairs >= 100000000ull ? 16 : crowd_pairs >= 40000000ull ? 8 : crowd_pairs >= 15000000ull ? 4 : per);
+}
+
 constexpr int kCellBlock = 128;  // threads of k_cells: a small population's cells spread over all SMs
 constexpr int kCellWarps = kCellBlock / 32;
 constexpr int kCellBlocksPerSm = 8;
@@ -3582,7 +3597,7 @@ __global__ void __launch_bounds__(kCellBlock, kCellBlocksPerSm) k_cells(StepArgs
     const int per_warp = max(8, min(32, (nc + warps - 1) / warps));
     if (per_warp * static_cast<int>(blockIdx.x * kCellWarps) >= nc) return;
     const PairGate pg = pair_gate(a);
-    const int per = f.per;
+    const int per = f.lift ? lifted_per(f.per, ctrl->crowd_pairs) : f.per;
     int2* span = hit_span[warp];
     unsigned short* tag = hit_tag[warp];
     unsigned long long cand = 0;
@@ -4331,6 +4346,7 @@ void launch_count_cells(const DeviceBuffers& b, const StepArgs& a, bool screen, 
     f.items = set.items;
     f.items_cap = b.items_cap;
     f.per = item_blocks(a.tune, a.n, !a.beside);
+    f.lift = a.tune.item_col_blocks == 0 && a.n < (1 << 17);
     f.runs = a.n >= (1 << 17);
     const bool o = a.overlap != 0;
     launch_after(o && !screen && !a.aside, screen ? k_place<true> : k_place<false>, grid_for(a.n, 8), kBlock, stream, a, f,
