@@ -258,6 +258,7 @@ struct StepArgs {
     float4* rec32;             // FP32 record of each object, written with its key (object order)
     int order;                 // counted build: crowded cells are put in sub-cell order
     int dense;                 // cells are built by sorting although they could be counted
+    int refine_early;          // the refinement is launched while the tile kernel drains
     int overlap;               // the step's kernels may start while their predecessors drain (launch_after)
     int pack_bits;             // > 0: sort keys carry the object index in their low pack_bits bits
     // Fragmentation on the device (null / 0 otherwise): the live population

@@ -4390,10 +4390,11 @@ namespace {
 // the states to the end. us a step, so / in stream order: 250 000 objects a
 // day old within 50 km (0.75M pairs refined) 548 / 483, a million within 20 km
 // (2M) 1272 / 1195, within 50 km (14M) 7602 / 6275; few pairs the same (a catalogue 34.1 / 33.3).
+// Small one-shot calls do (a.refine_early): the launch is 2-3% of them (2 111 objects 108.2 / 111.8 us).
 void refine(const DeviceBuffers& b, const StepArgs& a, const double* after, const double* size_m, bool by_pair,
             ks_conjunction* conj_out, int64_t conj_cap, ChunkCtrl* chunk, cudaStream_t stream) {
-    (by_pair ? k_refine_exact<true> : k_refine_exact<false>)<<<sm_count() * 2, kBlock, 0, stream>>>(
-        a, b.state[a.src], after, size_m, set_of(b, a).survivors, b.surv_cap, conj_out, conj_cap, chunk);
+    launch_after(a.refine_early != 0, by_pair ? k_refine_exact<true> : k_refine_exact<false>, sm_count() * 2, kBlock, stream, a,
+                 b.state[a.src], after, size_m, set_of(b, a).survivors, b.surv_cap, conj_out, conj_cap, chunk);
 }
 }  // namespace
 
