@@ -45,7 +45,8 @@ def test_tuning_without_screening_times_the_steps_a_run_takes(ks, oracle, block)
         eng.set_tuning("prop_block", block)
         eng.set_population(st, sz, al)
         choice = eng.autotune(130)
-        assert choice["trials"] == 1 + sum(v != block for v in (64, 96, 128))
+        # The start and the block sizes; a starting size among them is tried again where another has beaten it.
+        assert choice["trials"] - 1 in ((3,) if block == 32 else (2, 3))
         assert choice["steps_per_graph"] == 0
         assert eng.clock() == (0.0, 0) and len(eng.take_step_stats()) == 0
         eng.set_tuning("prop_block", block)
