@@ -105,6 +105,7 @@ struct ks_ctx {
     bool pairs_known = false;  // there was such a step
     bool dense = false;        // cells are built by sorting (sort_pays)
     bool one_stream = false;   // refinement outweighs the rest (plan_build)
+    bool refine_early = false; // beside the next step it is launched while the tile kernel drains (plan_build)
     bool crowded = false;      // crowded cells are put in order (order_pays)
     bool conj_small = false;   // chunks order their records in one launch (few expected)
     int64_t chunk_spec = 0;    // records a chunk copies back with its control blocks
@@ -682,7 +683,7 @@ void record_chunk_end(ks_ctx* ctx, bool capturing) {
 // buffers, its cells and its list of pairs to stay as they are meanwhile: a
 // third state buffer and a second set of the rest. Not with fragmentation on
 // the device, which follows the refinement inside the step, nor with per-phase
-// timing. In us a step, in one stream / refinement aside / pairs too:
+// timing, nor where refinement outweighs the rest (plan_build). In us a step, in one stream / refinement aside / pairs too:
 // catalogue hour 46.7 / 42.4 / 38.8, at dt 60 s 57.7 / 51.3 / 44.9, 250 000
 // objects 192 / 176 / 160, a million (split) 465 / 450 / 408. (A higher priority for
 // either stream: 250 000 objects 168 -> 186 or 175.)
@@ -718,10 +719,13 @@ std::vector<int> state_turns(ks_ctx* ctx, int k_steps, int src0) {
 // read the keys and records it replaces, its cell build for the propagation
 // and for the pairs that used its set two steps ago, its pairs for the cells.
 // The propagation shares the cell build's stream at sizes where its blocks,
-// which fill the chip for longer than a cell kernel takes, only displace that
-// build (250 000 objects 165 us a step, on a stream of its own 178; catalogue
-// hour 38.9 and 35.1, dt 60 s 45.2 and 41.1, a million FP64 427 and 406, split
-// 381 and 366, the ensemble 732 and 706).
+// which fill the chip for longer than a cell kernel takes, may only displace that
+// build. us a step, shared / on a stream of its own: catalogue hour 38.9 / 35.1, dt
+// 60 s 45.2 / 41.1, a million FP64 427 / 406, split 381 / 366, the ensemble 732 / 706; between
+// the lines chunks launched without a graph decide: 250 000 objects at dt 30 s 165 / 178, at
+// 60 s 441 / 474, 150 000 at 60 s 203 / 219 (at 10 s 99 / 97). Graphs prefer a stream of its own
+// there too (200 000 at 10 s 109 / 99, 400 000 178 / 160, 250 000 at 30 s 173 / 158), except in
+// batches (5 catalogues 106 / 113).
 void enqueue_aside(ks_ctx* ctx, int k_steps, int src0) {
     const bool own = ctx->n < (1 << 17) || ctx->n >= (1 << 19);
     cudaStream_t s = ctx->stream, p = own ? ctx->ahead : s, d = ctx->side;
@@ -736,6 +740,7 @@ void enqueue_aside(ks_ctx* ctx, int k_steps, int src0) {
         StepArgs a = step_args(ctx, k, k_steps, buf[k], buf[k + 1]);
         a.aside = own;
         a.beside = 1;
+        a.refine_early = ctx->refine_early;
         a.odd = k & 1;
         if (a.odd) a.rec32 = ctx->b.second.rec32;
         StepArgs alone = a;   // for kernels that follow an event of another stream
@@ -1007,14 +1012,24 @@ bool sort_pays(ks_ctx* ctx, bool streams) {
 // with their shared memory (refine). us a step, beside / in one stream, by refined pairs per
 // object: 8 (600 000 objects) 1925 / 1907, 14 (a million) 6275 / 6534, 18 (100 000) 691 / 680, 30 (250 000)
 // 1999 / 2046, 70 (60 000) 1451 / 1158, 138 (100 000) 3866 / 3231, 222 (60 000) 4240 / 3316.
+// Beside the next step a large population's pairs and refinements are the longest of the
+// streams, and an early launch of the refinement (refine) saves more than the L1 cache
+// while few pairs are refined: in stream order / early, 800 000 objects with 0.04 an object
+// 295.2 / 293.5, a million with 0.05 386.6 / 384.7 (360 steps end to end 125.2 / 124.2 ms), 450 000 with 0.7
+// 341 / 329; with 11 (800 000) 2858 / 3617, 3.5 (two million) 3881 / 4184, without any (a million, 0.002) 326.4 / 331.6;
+// 250 000 with 0.01 114.2 / 115.6, in one stream a million with 0.07 433 / 439.
 void plan_build(ks_ctx* ctx, bool streams) {
     if (!ctx->screening) return;
     const bool one = ctx->pairs_known && ctx->refined_each >= (ctx->one_stream ? 32.0 : 40.0);
     const bool dense = sort_pays(ctx, streams && !one);
-    if (one == ctx->one_stream && dense == ctx->dense) return;
+    const double slack = ctx->refine_early ? 2.5 : 1.0;  // clouds that spread and meet again change it often
+    const bool early = streams && !one && !dense && ctx->pairs_known && ctx->n >= kOrderObjects &&
+                       ctx->refined_each * slack >= 0.005 && ctx->refined_each < slack;
+    if (one == ctx->one_stream && dense == ctx->dense && early == ctx->refine_early) return;
     ctx->one_stream = one;
     ctx->dense = dense;
-    drop_graphs(ctx);  // they hold both
+    ctx->refine_early = early;
+    drop_graphs(ctx);  // they hold all three
 }
 
 // Whether a run whose density no step has shown yet may be one of those: its

@@ -3175,10 +3175,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sort_cells(StepArgs a, Fus
 // step and take 27 + 6; a batch of 64 such populations (2.13M objects, too
 // many for the cooperative sort's registers) 766 + 1400 us, now 400 + 365.
 // Every launch is bound by the latency of its few dependent L2 accesses at
-// small n and by L2 atomics and random sectors at large n (4-5% of DRAM). With
+// small n and by L2 round trips, atomics and random sectors at large n (cold, at
+// 400 000 objects: k_place 3% of DRAM, k_number 6%, k_scatter 21%, k_cells 3%). With
 // 1M objects in 88 000 cells the builds are closer (104 against 125 us), and
 // the tile kernel takes longer (222 against 208: objects arrive in a cell in no
-// spatial order).
+// spatial order). Steps of many more pairs have their cells sorted (sort_pays).
 // ---------------------------------------------------------------------------
 
 // Candidate pairs up to which a cell is screened by its own lanes.
@@ -3222,7 +3223,10 @@ __device__ __forceinline__ unsigned long long fib_slot(unsigned long long key, i
 // kernel reads, and a cell's lookups meet in few sectors (4M objects: cell
 // build 357 -> 306 us, pairs 880 -> 863; a million 107 -> 104). A small
 // population's cells spread evenly instead: crowded runs cost retries, and all
-// its objects wait for the unluckiest (28 340 objects: 29 us, in runs 39).
+// its objects wait for the unluckiest (28 340 objects: 29 us, in runs 39). A step
+// spread evenly / in runs near the line, us: 131 000 objects at dt 10 s 67 / 77, at 30 s 80 / 79,
+// 262 000 120 / 127 and 183 / 183, 8 catalogues in a batch 96 / 137, 24 catalogues 225 / 310, 600 000 231 / 231,
+// a million 415 / 406: the line lies low for sparse populations of this size.
 __device__ __forceinline__ unsigned long long home_bucket(const CountArgs& f, unsigned long long key) {
     if (!f.runs) return fib_slot(key, f.shift);
     return (fib_slot(key >> 5, f.shift + 3) << 3) | ((key >> 2) & 7);
@@ -4389,8 +4393,9 @@ namespace {
 // still divided for that kernel's shared memory and keep a small L1 cache for
 // the states to the end. us a step, so / in stream order: 250 000 objects a
 // day old within 50 km (0.75M pairs refined) 548 / 483, a million within 20 km
-// (2M) 1272 / 1195, within 50 km (14M) 7602 / 6275; few pairs the same (a catalogue 34.1 / 33.3).
-// Small one-shot calls do (a.refine_early): the launch is 2-3% of them (2 111 objects 108.2 / 111.8 us).
+// (2M) 1272 / 1195, within 50 km (14M) 7602 / 6275, a catalogue 34.1 / 33.3. With a.refine_early it is:
+// small one-shot calls, 2-3% of which the launch is (2 111 objects 108.2 / 111.8 us), and steps that
+// plan_build names.
 void refine(const DeviceBuffers& b, const StepArgs& a, const double* after, const double* size_m, bool by_pair,
             ks_conjunction* conj_out, int64_t conj_cap, ChunkCtrl* chunk, cudaStream_t stream) {
     launch_after(a.refine_early != 0, by_pair ? k_refine_exact<true> : k_refine_exact<false>, sm_count() * 2, kBlock, stream, a,
