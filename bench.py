@@ -390,8 +390,10 @@ def roofline_of(tm, a, fp64_rate, fp32_rates, split):
             # How busy the pipes really are (the pair kernel prunes most candidates
             # before its gate, so the algorithmic rate above can near the issue rate).
             "pipes_ncu": pipes_of(dom, split),
-            "pipes_ncu_source": "ncu --set full of one launch at 400k objects (the committed profile summaries), "
-                                "not measured in this run",
+            "pipes_ncu_source": "ncu --set full of one launch at 400k objects with cells built by counting (the "
+                                "committed profile summaries), not measured in this run",
+            "traffic_source": "ncu, DRAM bytes of one launch at 1M objects with cells built by counting, steps in "
+                              "one stream (profiles/traffic_per_launch.txt), not measured in this run",
             "peak_source": "measured on this GPU by the project microbenchmarks (dependent chains of FP32 add/mul, "
                            "FMA and packed FFMA2, FP64 add/mul; the highest FP32 rate is the peak); "
                            "MEASURED_PEAKS.json has no FP64/FP32 SIMT figure",
@@ -591,6 +593,8 @@ def main():
                  "over": f"the {a.steps} timed steps, pairs matched by (i, j, step)"},
                 **borderline_pairs(c_head, c_other, sz, a.conj_km, head == ks.PRECISION_SPLIT)),
             "refined_pairs_per_step": main_s["refined_pairs_per_step"],
+            "timed_route": "steps in one stream: events between their phases and an L2 flush between steps; a run "
+                           "without either overlaps neighbouring steps (e2e)",
             "wall_s_timed_region": main_s["wall_s_timed_region"]}
     if not a.no_error_study:
         line["split_error_vs_fp64"] = error_study(ks, eng, a, st, al)
