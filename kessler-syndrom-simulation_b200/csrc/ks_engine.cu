@@ -105,7 +105,7 @@ struct ks_ctx {
     bool pairs_known = false;  // there was such a step
     bool dense = false;        // cells are built by sorting (sort_pays)
     bool one_stream = false;   // refinement outweighs the rest (plan_build)
-    bool refine_early = false; // beside the next step it is launched while the tile kernel drains (plan_build)
+    bool refine_early = false; // it is launched while the tile kernel drains (plan_build)
     bool crowded = false;      // crowded cells are put in order (order_pays)
     bool conj_small = false;   // chunks order their records in one launch (few expected)
     int64_t chunk_spec = 0;    // records a chunk copies back with its control blocks
@@ -784,7 +784,8 @@ void enqueue_chunk(ks_ctx* ctx, int k_steps, int src0, bool capturing) {
     } else {
         int src = src0;
         for (int k = 0; k < k_steps; ++k) {
-            const StepArgs a = step_args(ctx, k, k_steps, src);
+            StepArgs a = step_args(ctx, k, k_steps, src);
+            a.refine_early = a.overlap && ctx->refine_early;
             record(ctx, k, 6, capturing);
             if (ctx->l2_flush_bytes > 0) cudaMemsetAsync(ctx->l2_flush, k & 0xFF, ctx->l2_flush_bytes, s);
             record(ctx, k, 0, capturing);
@@ -1017,14 +1018,16 @@ bool sort_pays(ks_ctx* ctx, bool streams) {
 // while few pairs are refined: in stream order / early, 800 000 objects with 0.04 an object
 // 295.2 / 293.5, a million with 0.05 386.6 / 384.7 (360 steps end to end 125.2 / 124.2 ms), 450 000 with 0.7
 // 341 / 329; with 11 (800 000) 2858 / 3617, 3.5 (two million) 3881 / 4184, without any (a million, 0.002) 326.4 / 331.6;
-// 250 000 with 0.01 114.2 / 115.6, in one stream a million with 0.07 433 / 439.
+// 250 000 with 0.01 114.2 / 115.6. In one stream the launch weighs more than the cache below 0.05 (58 650 objects
+// with fragmentation on the device, 13 steps 1373 / 1348 us; 33 000 with 0.5 an object 111.8 / 114.4 a step, a million with 0.07 433 / 439).
 void plan_build(ks_ctx* ctx, bool streams) {
     if (!ctx->screening) return;
     const bool one = ctx->pairs_known && ctx->refined_each >= (ctx->one_stream ? 32.0 : 40.0);
     const bool dense = sort_pays(ctx, streams && !one);
     const double slack = ctx->refine_early ? 2.5 : 1.0;  // clouds that spread and meet again change it often
-    const bool early = streams && !one && !dense && ctx->pairs_known && ctx->n >= kOrderObjects &&
-                       ctx->refined_each * slack >= 0.005 && ctx->refined_each < slack;
+    const bool early = !one && !dense &&
+                       (streams ? ctx->n >= kOrderObjects && ctx->refined_each * slack >= 0.005 && ctx->refined_each < slack
+                                : ctx->refined_each < 0.05 * slack);
     if (one == ctx->one_stream && dense == ctx->dense && early == ctx->refine_early) return;
     ctx->one_stream = one;
     ctx->dense = dense;
