@@ -78,3 +78,23 @@ def test_dense_steps_with_fragmentation(ks, dense, device):
     same(got, want)
     for f in EVENT_FIELDS:
         assert np.array_equal(events[f], want_events[f]), f
+
+
+@pytest.mark.parametrize("n,dt,chunks,form", [
+    (270_000, 120.0, [1, 7], 1),    # crowded cells could be put in order by then: 4 500 pairs an object decide
+    (2_000_000, 25.0, [1, 3], 0),   # too many for the cooperative sort: the separate kernels
+])
+def test_dense_steps_of_larger_populations(ks, n, dt, chunks, form):
+    st, sz, al = ks.generate_population(43, 28340, n, 200, 86400.0)
+    got = []
+    for fused in (2, 0):
+        with configured(ks, 3, dt) as eng:
+            eng.set_precision(ks.PRECISION_SPLIT)
+            eng.set_tuning("sort_fused", fused)
+            eng.set_population(st, sz, al)
+            for k in chunks:
+                eng.run(k)
+            assert eng.timing()["sort_cells_fused"] == (form if fused == 2 else 0)
+            got.append(results(eng))
+    assert got[1][3]["candidate_pairs"].min() > (4500 if form else 2000) * n
+    same(*got)
